@@ -36,6 +36,7 @@
 #include "mr_lengths.hpp"
 #include "pb_aux.hpp"
 #include "pencil_b200.h"
+#include "rx_plan.hpp"
 
 namespace pb {
 
@@ -996,6 +997,10 @@ static LocalOp local_op(const Stage& st, int mode, long long n_axis) {
 static int choose_lines_capped(pb_plan& P, PassArgs& A, int pair_kind, int cap);
 
 // Shape key of a generic pass (the autotuner's cache key).
+static cudaError_t launch_step(const PassArgs& A, int real_bytes, cudaStream_t stream) {
+  return A.fast == 5 ? launch_rx(A, real_bytes, stream) : launch_pass(A, real_bytes, stream);
+}
+
 static std::string pass_key(const PassArgs& A, int real_bytes) {
   return "k" + std::to_string(A.kind) + "s" + std::to_string(A.sub) + "n" + std::to_string(A.n_in) + "o" +
          std::to_string(A.n_out) + "m" + std::to_string(A.m) + "r" + std::to_string(real_bytes) + "c" +
@@ -1032,16 +1037,75 @@ static int choose_lines_capped(pb_plan& P, PassArgs& A, int pair_kind, int cap) 
   }
 }
 
+static int device_sms() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Per-stage twiddle vectors of the runtime-radix kernel, gathered from the
+// m-th roots.
+static size_t rx_table(pb_plan& P, const PassArgs& A) {
+  const std::vector<int> rad(A.radix, A.radix + A.nstages);
+  std::string key = "X";
+  for (int r : rad) key += "_" + std::to_string(r);
+  auto it = P.cache.find(key);
+  if (it != P.cache.end()) return it->second;
+  const size_t roots = roots_table(P, A.m);
+  size_t off;
+  if (P.real_bytes == 4) {
+    const std::vector<float> t = rx_twiddles<float>(rad, reinterpret_cast<const float*>(&P.host.bytes[roots]));
+    off = P.host.add(t.data(), t.size() * sizeof(float));
+  } else {
+    const std::vector<double> t = rx_twiddles<double>(rad, reinterpret_cast<const double*>(&P.host.bytes[roots]));
+    off = P.host.add(t.data(), t.size() * sizeof(double));
+  }
+  P.cache[key] = off;
+  return off;
+}
+
+// Persistent grid of a register kernel: its resident CTAs on every SM.
+static void set_grid(const pb_plan& P, PassArgs& A) {
+  if (A.fast && !P.force_generic) {
+    const int occ = A.fast == 5   ? rx_occupancy(A, P.real_bytes)
+                    : A.fast == 4 ? mr_bs_occupancy(A.bs_m2, A.kind, mr_bs_variant(A), P.real_bytes)
+                    : A.fast == 3 ? mr_r2r_occupancy(A.m, P.real_bytes)
+                    : A.fast == 2 ? mr_occupancy(A.m, P.real_bytes)
+                    : A.half      ? pow2_half_occupancy(A.m, A.kind)
+                                  : pow2_occupancy(A.m, A.kind, A.inv, A.dst_k_contig == 1, P.real_bytes);
+    A.grid_ctas = device_sms() * std::max(1, occ);
+  }
+}
+
 // Tile, piece and k tables of the register kernel, in the tile order of the
 // generic kernel: tile = ((e * outer) + outer_index) * nchunks + chunk.
 static void build_fast_tables(pb_plan& P, PassArgs& A, const Pencil& src, const Pencil& dst,
                               const std::vector<int2>& chunks) {
-  HostLayout hs(src, P.extra), hd(dst, P.extra);
   const int N = src.N;
   const bool direct = A.dst_k_contig == 1;  // 2: direct store split into pieces
   const int ta = dst.split_of(A.a);
   const int npieces = direct ? 1 : (ta >= 0 ? dst.grid[ta] : 1);
   const long long nout = dst.shape[A.a];
+  // the operations of a plan share most of their passes' layouts: equal tables
+  // are built once
+  std::string key;
+  if (!P.sliced) {
+    key = "T" + pencil_key(src, P.extra) + pencil_key(dst, P.extra) + "a" + std::to_string(A.a) + "b" +
+          std::to_string(A.b) + "l" + std::to_string(A.lines) + "k" + std::to_string(A.src_k_contig) +
+          std::to_string(A.dst_k_contig) + "h" + std::to_string(A.half);
+    auto it = P.cache.find(key);
+    if (it != P.cache.end()) {
+      A.tile_tab = enc(it->second);
+      if (!direct) {
+        A.piece_tab = enc(P.cache.at(key + "p"));
+        A.ktab = reinterpret_cast<const int2*>(enc(P.cache.at(key + "k")));
+      }
+      A.npieces = npieces;
+      set_grid(P, A);
+      return;
+    }
+  }
+  HostLayout hs(src, P.extra), hd(dst, P.extra);
   std::vector<TileAddr> tiles((size_t)A.ntiles);
   std::vector<PieceAddr> pieces(direct ? 0 : (size_t)A.ntiles * npieces);
   // a slice keeps the tiles whose lines lie in its ranks, with addresses from
@@ -1108,28 +1172,30 @@ static void build_fast_tables(pb_plan& P, PassArgs& A, const Pencil& src, const 
     if (!direct) pieces.resize((size_t)t * npieces);
     A.ntiles = t;
   }
-  A.tile_tab = enc(P.host.add(tiles.data(), tiles.size() * sizeof(TileAddr)));
+  const size_t tile_off = P.host.add(tiles.data(), tiles.size() * sizeof(TileAddr));
+  size_t piece_off = 0, k_off = 0;
+  A.tile_tab = enc(tile_off);
   if (!direct) {
-    A.piece_tab = enc(P.host.add(pieces.data(), pieces.size() * sizeof(PieceAddr)));
+    piece_off = P.host.add(pieces.data(), pieces.size() * sizeof(PieceAddr));
+    A.piece_tab = enc(piece_off);
     std::vector<int2> kt((size_t)nout);
     for (long long k = 0; k < nout; ++k) {
       const int p = (npieces > 1) ? (int)(((k + 1) * npieces - 1) / nout) : 0;
       kt[(size_t)k].x = p;
       kt[(size_t)k].y = (int)(k - Pencil::part(nout, npieces, p));
     }
-    A.ktab = reinterpret_cast<const int2*>(enc(P.host.add(kt.data(), kt.size() * sizeof(int2))));
+    k_off = P.host.add(kt.data(), kt.size() * sizeof(int2));
+    A.ktab = reinterpret_cast<const int2*>(enc(k_off));
   }
   A.npieces = npieces;
-  if (A.fast && !P.force_generic) {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int occ = A.fast == 4   ? mr_bs_occupancy(A.bs_m2, A.kind, mr_bs_variant(A), P.real_bytes)
-                    : A.fast == 3 ? mr_r2r_occupancy(A.m, P.real_bytes)
-                    : A.fast == 2 ? mr_occupancy(A.m, P.real_bytes)
-                    : A.half      ? pow2_half_occupancy(A.m, A.kind)
-                                  : pow2_occupancy(A.m, A.kind, A.inv, A.dst_k_contig == 1, P.real_bytes);
-    A.grid_ctas = sms * std::max(1, occ);
+  if (!P.sliced) {
+    P.cache[key] = tile_off;
+    if (!direct) {
+      P.cache[key + "p"] = piece_off;
+      P.cache[key + "k"] = k_off;
+    }
   }
+  set_grid(P, A);
 }
 
 // One fused pass for `st` under `op` from layout `src` to layout `dst`.
@@ -1208,6 +1274,15 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
   A.dst_k_contig = (dst.perm[N - 1] == a) ? 1 : 0;
   const bool pair_kind = (op.kind == P_R2C || op.kind == P_C2R || (op.kind == P_R2R && !in_complex));
   int L = 0;
+  // the tile axis is cut at both partitions of axis b
+  std::vector<long long> cuts{0, src.shape[b]};
+  for (const Pencil* p : {&src, &dst}) {
+    const int t = p->split_of(b);
+    if (t >= 0)
+      for (int c = 1; c < p->grid[t]; ++c) cuts.push_back(Pencil::part(p->shape[b], p->grid[t], c));
+  }
+  std::sort(cuts.begin(), cuts.end());
+  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
   // register-resident power-of-two kernel: lines contiguous in one source rank,
   // destination either with the same property (direct) or with the tile axis
   // innermost and unsplit (transposed store)
@@ -1296,6 +1371,30 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
       A.lines = L;
     }
   }
+  // every other length with prime factors up to 31, any kind: the
+  // runtime-radix kernel, on the same layouts (the split direct store for
+  // every kind)
+  if (!A.fast && !P.force_generic && op.kind != P_COPY && !A.bs_m2 && (src.perm[N - 1] == a || r2r_strided) &&
+      src.split_of(a) < 0) {
+    const int ta = dst.split_of(a);
+    const bool direct = dst.perm[N - 1] == a && ta < 0;
+    const bool transposed = !direct && dst.perm[N - 1] == b && (ta < 0 || dst.grid[ta] <= kRxMaxPieces);
+    const bool dsplit = !direct && dst.perm[N - 1] == a && ta >= 0 && dst.grid[ta] <= kRxMaxPieces;
+    if (direct || transposed || dsplit) {
+      PassArgs B = A;
+      B.dst_k_contig = direct ? 1 : (dsplit ? 2 : 0);
+      long long run = 0, lines = P.extra;
+      for (size_t i = 0; i + 1 < cuts.size(); ++i) run = std::max(run, cuts[i + 1] - cuts[i]);
+      for (int x = 0; x < N; ++x)
+        if (x != a) lines *= src.shape[x];
+      if (rx_choose(B, P.real_bytes, P.max_smem, run, lines, device_sms())) {
+        A = B;
+        A.fast = 5;
+        A.twiddle = enc(rx_table(P, A));
+        L = A.lines;
+      }
+    }
+  }
   // inside the persistent batch kernel: its mixed-radix tiles (f32, 7-smooth
   // lengths up to 256), same layout conditions
   if (!A.fast && P.force_generic && P.batch_mr && (op.kind == P_C2C || op.kind == P_R2C || op.kind == P_C2R) &&
@@ -1313,7 +1412,7 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
   // the register kernels' row tables hold A.m outputs per line
   // (mr_r2r_table_len in the real-to-real kernel): anything longer stays on
   // the generic kernel
-  if (A.fast && A.n_out > (A.fast == 3 ? mr_r2r_table_len(A.m) : (A.half ? 2 * A.m : A.m))) {
+  if (A.fast && A.fast != 5 && A.n_out > (A.fast == 3 ? mr_r2r_table_len(A.m) : (A.half ? 2 * A.m : A.m))) {
     A.fast = 0;
     A.half = 0;
     A.m = fft_len(op.kind, op.sub, A.n);
@@ -1325,15 +1424,6 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
     auto it = P.tuned_lines.find(pass_key(A, P.real_bytes));
     if (it != P.tuned_lines.end() && it->second < L) L = choose_lines_capped(P, A, pair_kind ? 1 : 0, it->second);
   }
-  // chunks of the tile axis, split at both partitions of axis b
-  std::vector<long long> cuts{0, src.shape[b]};
-  for (const Pencil* p : {&src, &dst}) {
-    const int t = p->split_of(b);
-    if (t >= 0)
-      for (int c = 1; c < p->grid[t]; ++c) cuts.push_back(Pencil::part(p->shape[b], p->grid[t], c));
-  }
-  std::sort(cuts.begin(), cuts.end());
-  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
   std::vector<int2> chunks;
   for (size_t i = 0; i + 1 < cuts.size(); ++i)
     for (long long j = cuts[i]; j < cuts[i + 1]; j += L) {
@@ -1812,7 +1902,7 @@ static int run(pb_plan* P, int op, const void* in, void* out, void* ws, cudaStre
       A.in = slot_ptr(*P, st.src_slot, in, out, ws);
       A.out = slot_ptr(*P, st.dst_slot, in, out, ws);
       A.gate = (A.gate != nullptr) ? status : nullptr;
-      cuda_ok(launch_pass(A, P->real_bytes, s));
+      cuda_ok(launch_step(A, P->real_bytes, s));
     } else {
       StatsArgs S = st.sa;
       S.data = slot_ptr(*P, st.src_slot, in, out, ws);
@@ -2166,7 +2256,7 @@ int pb_plan_step_kernels(const pb_plan* plan, int32_t op, int32_t* kernels, int3
     const Program& prog = plan->prog[user_mode(*plan, op)];
     int n = 0;
     for (const Step& s : prog.steps) {
-      const int k = s.type != 0 ? 1 : (s.pa.fast == 1 ? 2 : (s.pa.fast == 4 ? 4 : (s.pa.fast >= 2 ? 3 : 0)));
+      const int k = s.type != 0 ? 1 : (s.pa.fast == 1 ? 2 : (s.pa.fast >= 4 ? s.pa.fast : (s.pa.fast >= 2 ? 3 : 0)));
       if (kernels && n < capacity) kernels[n] = k;
       ++n;
     }
@@ -3329,9 +3419,9 @@ static void autotune_pass(pb_plan& T, const pb_plan& plan, int mode, int step, v
     st.pa.in = scratch_a;
     st.pa.out = scratch_b;
     st.pa.gate = nullptr;
-    cuda_ok(launch_pass(st.pa, T.real_bytes, 0));
+    cuda_ok(launch_step(st.pa, T.real_bytes, 0));
     cuda_ok(cudaEventRecord(e0, 0));
-    for (int r = 0; r < 3; ++r) cuda_ok(launch_pass(st.pa, T.real_bytes, 0));
+    for (int r = 0; r < 3; ++r) cuda_ok(launch_step(st.pa, T.real_bytes, 0));
     cuda_ok(cudaEventRecord(e1, 0));
     cuda_ok(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -4153,7 +4243,7 @@ static int slice_phase(pb_slice& S, int op, int phase, const void* in, void* out
       check_aligned(A.in, A.in_complex != 0, P.real_bytes);
       check_aligned(A.out, A.out_complex != 0, P.real_bytes);
       A.gate = (A.gate != nullptr) ? status : nullptr;
-      cuda_ok(launch_pass(A, P.real_bytes, s));
+      cuda_ok(launch_step(A, P.real_bytes, s));
     } else if (st.type == 1) {
       StatsArgs St = st.sa;
       St.data = slice_slot(S, st.src_slot, in, out, ws);
@@ -4307,7 +4397,8 @@ static std::string reg_key(const PassArgs& A, int real_bytes) {
 }
 
 static int reg_occupancy(const PassArgs& A, int real_bytes, int sched) {
-  return A.fast == 4   ? mr_bs_occupancy(A.bs_m2, A.kind, mr_bs_variant(A), real_bytes)
+  return A.fast == 5   ? rx_occupancy(A, real_bytes)
+         : A.fast == 4 ? mr_bs_occupancy(A.bs_m2, A.kind, mr_bs_variant(A), real_bytes)
          : A.fast == 3 ? mr_r2r_occupancy(A.m, real_bytes)
          : A.fast == 2 ? mr_occupancy(A.m, real_bytes, sched)
          : A.half      ? pow2_half_occupancy(A.m, A.kind)
@@ -4379,12 +4470,12 @@ static int autotune_plan(pb_plan* plan) {
           A.sched = sc;
           A.grid_ctas = sms * c;
           float ms = 0.f;
-          if (launch_pass(A, P.real_bytes, 0) != cudaSuccess || cudaEventRecord(e0, 0) != cudaSuccess) {
+          if (launch_step(A, P.real_bytes, 0) != cudaSuccess || cudaEventRecord(e0, 0) != cudaSuccess) {
             rc = PB_ECUDA;
             break;
           }
           for (int r = 0; r < 3; ++r)
-            if (launch_pass(A, P.real_bytes, 0) != cudaSuccess) rc = PB_ECUDA;
+            if (launch_step(A, P.real_bytes, 0) != cudaSuccess) rc = PB_ECUDA;
           if (rc != PB_OK || cudaEventRecord(e1, 0) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
               cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
             rc = PB_ECUDA;
@@ -4459,7 +4550,7 @@ int pb_plan_step_config(const pb_plan* plan, int32_t op, int32_t step, pb_step_c
     }
     const PassArgs& A = st.pa;
     const int sms = sm_count();
-    out->kernel = A.fast == 1 ? 2 : (A.fast == 2 || A.fast == 3) ? 3 : (A.fast == 4 ? 4 : 0);
+    out->kernel = A.fast == 1 ? 2 : (A.fast == 2 || A.fast == 3) ? 3 : (A.fast >= 4 ? A.fast : 0);
     out->fft_len = A.m;
     out->lines = A.lines;
     out->grid_ctas = A.fast ? (int)std::min<long long>(A.grid_ctas, A.ntiles) : 0;

@@ -1,0 +1,840 @@
+// Fused pass with stage radices chosen at run time, for the lengths that have
+// no compiled kernel of their own: C2C, R2C, C2R and the real-to-real kinds on
+// any length whose prime factors are at most 31.
+//
+// Persistent CTAs walk the pass's tiles.  The lines of the next tile are
+// copied to a staging area by cp.async while the current tile is transformed,
+// so no registers hold data in flight.  Two sequences (f32) or one (f64) form
+// a 16-byte vector, and a row buffer holds element i of all sequences of the
+// tile in row i: a butterfly reads and writes whole vectors, one twiddle, one
+// index computation and one packed instruction serve both sequences, and the
+// transposed store (the fused pencil transpose) reads its runs of the
+// destination's innermost axis directly.
+//
+//   first stage   staged lines -> butterfly -> rows (or, with `pre`, a pass
+//                 that forms the rows: the real-to-real kinds' reordering and
+//                 pre-twiddles, and lengths with a prime above 16)
+//   middle stages rows -> rows, alternating between two buffers
+//   last stage    C2C: butterfly outputs go to memory from registers; the
+//                 other kinds read the finished rows back (the Hermitian
+//                 split, post-twiddles) and store
+//
+// Inverse transforms read their input in reversed index order, X^-1[k] =
+// DFT(x[-q])[k], so only forward butterflies exist.
+//
+// What bounds it: shared-memory and barrier latency at 12 to 16 warps per SM,
+// not HBM (ncu, 384-point C2C f32: DRAM 55%, issue 45%, LSU data pipe 63%).
+// Against the generic kernel on the same passes (B200, forward + inverse):
+// 255^3 R2C f64 3.43 -> 1.11 ms, 4096^2 C2C f32 2.30 -> 0.63 ms; single
+// transposed C2C passes run at 2.4-3.9 TB/s.  Measured choices: tiles of about
+// 2000 points with 128 threads and four CTAs per SM beat tiles of twice the
+// lines with 256 threads (384 points: 3.9 against 3.1 TB/s); 80 registers and
+// more CTAs lose to 128 and fewer (3.8 against 3.9); loading straight into
+// registers instead of staging loses (3.3); twiddles from shared memory beat
+// global memory (2.8 against 2.4 TB/s at 1000 points) while they fit.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "pb_device.cuh"
+#include "rx_fft.cuh"
+#include "rx_plan.hpp"
+
+namespace pb {
+
+template <typename R>
+using RxV = VC<typename Vec<R>::Q>;
+
+template <int N>
+__device__ __forceinline__ void rx_cp_async(void* s, const void* g) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+  if constexpr (N == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(g) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(a), "l"(g), "n"(N) : "memory");
+}
+__device__ __forceinline__ void rx_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void rx_cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// vector (re, im) of W sequences from scalars
+__device__ __forceinline__ VC<Q2> rx_pack(float x0, float y0, float x1, float y1) {
+  return VC<Q2>{Q2{make_float2(x0, x1)}, Q2{make_float2(y0, y1)}};
+}
+
+// Copies one tile's lines into the staging area (line l, element q at
+// l*sl + q*sq).  E is the element type.  Lines run along the threads of a
+// group; 16-byte copies where the source row and the staging row allow it.
+template <typename E>
+__device__ __forceinline__ void rx_stage_lines(E* S, const RxArgs& X, const TileAddr& ta) {
+  constexpr int VF = 16 / (int)sizeof(E);
+  const PassArgs& A = X.p;
+  const RxGeom& g = X.g;
+  const int nt = blockDim.x, tid = threadIdx.x, n = A.n_in;
+  const E* in = reinterpret_cast<const E*>(A.in) + ta.src0;
+  if (A.src_k_contig) {
+    int lg = 31 - __clz(nt) - (31 - __clz(A.lines));
+    if (lg < 3) lg = 3;
+    const int tpl = 1 << lg, q0 = tid & (tpl - 1);
+    const bool srow = (g.sl & (VF - 1)) == 0;
+    for (int l = tid >> lg; l < ta.lines; l += nt >> lg) {
+      const E* p = in + (long long)l * ta.srcb;
+      E* s = S + l * g.sl;
+      int q = q0;
+      if (VF > 1 && srow && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        const int nv = n / VF;
+        for (; q < nv; q += tpl) rx_cp_async<16>(s + q * VF, p + q * VF);
+        q = nv * VF + q0;
+      }
+      for (; q < n; q += tpl) rx_cp_async<(int)sizeof(E)>(s + q, p + q);
+    }
+  } else {
+    const int nc = (A.lines + VF - 1) / VF;  // chunks of VF adjacent lines per element
+    const unsigned mc = fdiv_magic(nc);
+    const int total = n * nc;
+    for (int i = tid; i < total; i += nt) {
+      const int q = (int)fdiv(i, nc, mc), l = (i - q * nc) * VF;
+      const E* p = in + (long long)q * ta.srcq + (long long)l * ta.srcb;
+      E* s = S + q * g.sq + l;
+      if (VF > 1 && ta.srcb == 1 && l + VF <= ta.lines && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        rx_cp_async<16>(s, p);
+      } else {
+#pragma unroll
+        for (int j = 0; j < VF; ++j)
+          if (l + j < ta.lines) rx_cp_async<(int)sizeof(E)>(s + j, p + (long long)j * ta.srcb);
+      }
+    }
+  }
+  // the missing partner of an odd last line of a pair is zero
+  if ((A.kind == P_R2C || A.kind == P_C2R) && (ta.lines & 1)) {
+    E z;
+    memset(&z, 0, sizeof(E));
+    for (int q = tid; q < n; q += nt) S[ta.lines * g.sl + q * g.sq] = z;
+  }
+}
+
+template <typename R, int KIND>
+__device__ __forceinline__ void rx_stage(unsigned char* S, const RxArgs& X, const TileAddr& ta) {
+  using C = typename Cx<R>::T;
+  if (KIND == P_R2C || (KIND == P_R2R && !X.p.in_complex))
+    rx_stage_lines<R>(reinterpret_cast<R*>(S), X, ta);
+  else
+    rx_stage_lines<C>(reinterpret_cast<C*>(S), X, ta);
+}
+
+// FFT input of vector g at staging offset o (= element * sq): C2C lines, or
+// line pairs x + iy of real data.
+template <typename R, int KIND>
+__device__ __forceinline__ RxV<R> rx_fetch_at(const unsigned char* S, int base, int sl, int o) {
+  using C = typename Cx<R>::T;
+  if constexpr (KIND == P_C2C) {
+    const C* p = reinterpret_cast<const C*>(S) + base + o;
+    if constexpr (sizeof(R) == 4) {
+      const C a = p[0], b = p[sl];
+      return rx_pack(a.x, a.y, b.x, b.y);
+    } else {
+      const C a = p[0];
+      return RxV<R>{a.x, a.y};
+    }
+  } else {
+    const R* p = reinterpret_cast<const R*>(S) + base + o;
+    if constexpr (sizeof(R) == 4)
+      return rx_pack(p[0], p[sl], p[2 * sl], p[3 * sl]);
+    else
+      return RxV<R>{p[0], p[sl]};
+  }
+}
+
+// C2R: Hermitian extension X + iY of the half spectra of lines 2s and 2s + 1
+// at element q of the (index-reversed for a positive exponent) sequence.
+template <typename R>
+__device__ __forceinline__ RxV<R> rx_fetch_c2r(const unsigned char* S, const RxArgs& X, int g, int q) {
+  using C = typename Cx<R>::T;
+  const PassArgs& A = X.p;
+  const int m = A.m;
+  if (A.inv && q != 0) q = m - q;
+  const bool mirror = 2 * q > m;
+  const int hq = mirror ? m - q : q;
+  const bool edge = hq == 0 || 2 * hq == m;
+  const R w = (A.pre_mode == W_HALF_INTERIOR && !edge) ? R(A.pre_factor) : R(1);
+  const R sg = edge ? R(0) : (mirror ? -w : w);  // weight of the imaginary parts
+  const int sl = X.g.sl;
+  auto one = [&](int s, R& x, R& y) {
+    const C* p = reinterpret_cast<const C*>(S) + (2 * s) * sl + hq * X.g.sq;
+    const C a = p[0], b = p[sl];
+    const R ay = edge ? R(0) : a.y * sg, by = edge ? R(0) : b.y * sg;
+    x = a.x * w - by;
+    y = ay + b.x * w;
+  };
+  if constexpr (sizeof(R) == 4) {
+    R x0, y0, x1, y1;
+    one(2 * g, x0, y0);
+    one(2 * g + 1, x1, y1);
+    return rx_pack(x0, y0, x1, y1);
+  } else {
+    R x0, y0;
+    one(g, x0, y0);
+    return RxV<R>{x0, y0};
+  }
+}
+
+// lines of the staging area per vector
+template <typename R, int KIND>
+__device__ __forceinline__ constexpr int rx_lines_per_vec() {
+  return Vec<R>::W * (KIND == P_C2C ? 1 : 2);
+}
+
+// Stage 0 (no twiddles) from the staged lines.
+template <typename R, int KIND, int RAD>
+__device__ __forceinline__ void rx_first(const unsigned char* S, RxV<R>* out, const RxArgs& X) {
+  using Q = typename Vec<R>::Q;
+  const PassArgs& A = X.p;
+  const int m = A.m, NB = m / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
+  const int sl = X.g.sl, sq = X.g.sq;
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int g = it & ((1 << lgG) - 1), jb = it >> lgG;
+    RxV<R> v[RAD];
+    if constexpr (KIND == P_C2R) {
+#pragma unroll
+      for (int r = 0; r < RAD; ++r) v[r] = rx_fetch_c2r<R>(S, X, g, jb + r * NB);
+    } else {
+      // element jb + r*NB, or m - jb - r*NB (0 for element 0) when inverse
+      const int base = g * rx_lines_per_vec<R, KIND>() * sl;
+      const int b0 = (A.inv ? m - jb : jb) * sq, st = (A.inv ? -NB : NB) * sq;
+      v[0] = rx_fetch_at<R, KIND>(S, base, sl, (A.inv && jb == 0) ? 0 : b0);
+#pragma unroll
+      for (int r = 1; r < RAD; ++r) v[r] = rx_fetch_at<R, KIND>(S, base, sl, b0 + r * st);
+    }
+    VB<Q, RAD>::run(v);
+    RxV<R>* o = out + jb * RAD * P + g;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) o[r * P] = v[r];
+  }
+}
+
+// Rows from the staged lines without a stage (lengths whose stage 0 is a
+// direct-sum prime).
+template <typename R, int KIND>
+__device__ __forceinline__ void rx_rows(const unsigned char* S, RxV<R>* out, const RxArgs& X) {
+  const PassArgs& A = X.p;
+  const int m = A.m, lgG = X.g.lgG, P = X.g.P, total = m << lgG;
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int g = it & ((1 << lgG) - 1), q = it >> lgG;
+    if constexpr (KIND == P_C2R) {
+      out[q * P + g] = rx_fetch_c2r<R>(S, X, g, q);
+    } else {
+      const int e = (A.inv && q != 0) ? m - q : q;
+      out[q * P + g] = rx_fetch_at<R, KIND>(S, g * rx_lines_per_vec<R, KIND>() * X.g.sl, X.g.sl, e * X.g.sq);
+    }
+  }
+}
+
+// Stockham stage: butterfly jb (k = jb mod NS) takes rows jb + r*m/RAD times
+// W^{k r} and writes rows (jb - k)*RAD + k + r*NS.
+template <typename R, int RAD>
+__device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int NS, const RxV<R>* tw) {
+  using Q = typename Vec<R>::Q;
+  const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
+  const int rs = NB * P, ws = NS * P;
+  const unsigned mNS = fdiv_magic(NS);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int g = it & ((1 << lgG) - 1), jb = it >> lgG;
+    const int k = jb - (int)fdiv(jb, NS, mNS) * NS;
+    const RxV<R>* p = in + jb * P + g;
+    RxV<R> v[RAD];
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
+    if (NS > 1) {
+      const RxV<R>* t = tw + k;
+#pragma unroll
+      for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NS]);
+    }
+    VB<Q, RAD>::run(v);
+    RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) o[r * ws] = v[r];
+  }
+}
+
+// The same for a prime radix above kRxRegRadix: outputs h and RAD - h as
+// direct sums over the pairs (p, RAD - p) read from the rows, so no butterfly
+// sits in registers.  `roots` are the RAD-th roots.
+template <typename R>
+__device__ __forceinline__ void rx_mid_prime(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int RAD, int NS,
+                                             const RxV<R>* tw, const RxV<R>* roots) {
+  const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P;
+  const int H = (RAD - 1) / 2, total = (NB * (H + 1)) << lgG;
+  const int rs = NB * P, ws = NS * P;
+  const unsigned mNS = fdiv_magic(NS), mNB = fdiv_magic(NB);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int g = it & ((1 << lgG) - 1), b = it >> lgG;
+    const int h = (int)fdiv(b, NB, mNB), jb = b - h * NB;
+    const int k = jb - (int)fdiv(jb, NS, mNS) * NS;
+    const RxV<R>* p = in + jb * P + g;
+    const RxV<R> v0 = p[0];
+    RxV<R> a = v0, c = {qc<typename Vec<R>::Q>(0.0), qc<typename Vec<R>::Q>(0.0)};
+    int idx = 0;
+    for (int i = 1; i <= H; ++i) {
+      RxV<R> u = p[i * rs], w = p[(RAD - i) * rs];
+      if (NS > 1) {
+        u = vtw(u, tw[(i - 1) * NS + k]);
+        w = vtw(w, tw[(RAD - i - 1) * NS + k]);
+      }
+      idx += h;
+      if (idx >= RAD) idx -= RAD;
+      const RxV<R> t = roots[idx];  // (cos, -sin)
+      const RxV<R> s = vadd(u, w), d = vsub(u, w);
+      a = {qfma(s.x, t.x, a.x), qfma(s.y, t.x, a.y)};
+      c = {qfma(d.x, t.y, c.x), qfma(d.y, t.y, c.y)};
+    }
+    RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
+    // sum over d * (-i sin): a + i c with c carrying -sin
+    if (h == 0) {
+      o[0] = a;
+    } else {
+      o[h * ws] = vsubr(a, c);
+      o[(RAD - h) * ws] = vaddr(a, c);
+    }
+  }
+}
+
+// Destination of one tile: address of output k of line 0 and the line stride.
+struct RxDst {
+  int mode;  // 0 transposed, 1 direct, 2 direct split across the ranks
+  long long dst0;
+  int dstb;
+  const PieceAddr* prow;  // rows of the pieces, rebased to k = 0
+  int np, nout;
+  unsigned mnout;
+  int lines;
+  __device__ __forceinline__ const PieceAddr* piece(int k) const {
+    return prow + (np > 1 ? (int)fdiv((unsigned)((k + 1) * np - 1), nout, mnout) : 0);
+  }
+  __device__ __forceinline__ long long at(int k, int l) const {
+    if (mode == 1) return dst0 + (long long)l * dstb + k;
+    const PieceAddr* r = piece(k);
+    return mode == 0 ? r->rowbase + (long long)k * r->stride + l : r->rowbase + k + (long long)l * r->stride;
+  }
+};
+
+// two adjacent complex values
+__device__ __forceinline__ void rx_put2(float2* o, float2 a, float2 b, bool second) {
+  if (second && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+    *reinterpret_cast<float4*>(o) = make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    o[0] = a;
+    if (second) o[1] = b;
+  }
+}
+
+// Vector w of C2C results (output k of lines l .. l + W - 1) to memory.
+template <typename R>
+__device__ __forceinline__ void rx_put_c2c(typename Cx<R>::T* out, const RxDst& D, int k, int l, RxV<R> w) {
+  if constexpr (sizeof(R) == 4) {
+    const float2 a = make_float2(w.x.v.x, w.y.v.x), b = make_float2(w.x.v.y, w.y.v.y);
+    const long long o = D.at(k, l);
+    if (D.mode == 0) {
+      rx_put2(out + o, a, b, l + 1 < D.lines);
+    } else {
+      out[o] = a;
+      if (l + 1 < D.lines) out[D.at(k, l + 1)] = b;
+    }
+  } else {
+    out[D.at(k, l)] = make_double2(w.x, w.y);
+  }
+}
+
+// Last stage of a C2C pass, stored from registers.  Transposed: the lanes take
+// the vectors of a row, which are adjacent in the destination row; else
+// consecutive butterflies, whose outputs are adjacent in the destination line.
+template <typename R, int RAD, bool TR>
+__device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const RxV<R>* tw, const RxDst& D) {
+  using Q = typename Vec<R>::Q;
+  using C = typename Cx<R>::T;
+  const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
+  const int rs = NB * P;
+  const unsigned mNB = fdiv_magic(NB);
+  const Q sc = qc<Q>(X.p.scale);
+  C* out = reinterpret_cast<C*>(X.p.out);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    int g, jb;
+    if (TR) {
+      g = it & ((1 << lgG) - 1);
+      jb = it >> lgG;
+    } else {
+      g = (int)fdiv(it, NB, mNB);
+      jb = it - g * NB;
+    }
+    const int l = g * Vec<R>::W;
+    if (l >= D.lines) continue;
+    const RxV<R>* p = in + jb * P + g;
+    RxV<R> v[RAD];
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
+    const RxV<R>* t = tw + jb;
+#pragma unroll
+    for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NB]);
+    VB<Q, RAD>::run(v);
+    if (!TR && D.mode == 1) {
+      C* o = out + D.dst0 + (long long)l * D.dstb + jb;
+      const bool two = sizeof(R) == 4 && l + 1 < D.lines;
+#pragma unroll
+      for (int r = 0; r < RAD; ++r) {
+        const RxV<R> w = {qmul(v[r].x, sc), qmul(v[r].y, sc)};
+        if constexpr (sizeof(R) == 4) {
+          o[r * NB] = make_float2(w.x.v.x, w.y.v.x);
+          if (two) o[D.dstb + r * NB] = make_float2(w.x.v.y, w.y.v.y);
+        } else {
+          o[r * NB] = make_double2(w.x, w.y);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < RAD; ++r)
+        rx_put_c2c<R>(out, D, jb + r * NB, l, RxV<R>{qmul(v[r].x, sc), qmul(v[r].y, sc)});
+    }
+  }
+}
+
+// Work item of a store loop over n rows: lanes along the vectors of a row for
+// a transposed store, along the rows otherwise.
+__device__ __forceinline__ void rx_item(int it, int lgG, int n, unsigned mn, bool tr, int& g, int& k) {
+  if (tr) {
+    g = it & ((1 << lgG) - 1);
+    k = it >> lgG;
+  } else {
+    g = (int)fdiv(it, n, mn);
+    k = it - g * n;
+  }
+}
+
+// Finished rows to memory: C2C.
+template <typename R>
+__device__ __forceinline__ void rx_store_c2c(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
+  using Q = typename Vec<R>::Q;
+  const int n = X.p.m, lgG = X.g.lgG, total = n << lgG;
+  const unsigned mn = fdiv_magic(n);
+  const Q sc = qc<Q>(X.p.scale);
+  typename Cx<R>::T* out = reinterpret_cast<typename Cx<R>::T*>(X.p.out);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    int g, k;
+    rx_item(it, lgG, n, mn, D.mode == 0, g, k);
+    const int l = g * Vec<R>::W;
+    if (l >= D.lines) continue;
+    const RxV<R> v = rows[k * X.g.P + g];
+    rx_put_c2c<R>(out, D, k, l, RxV<R>{qmul(v.x, sc), qmul(v.y, sc)});
+  }
+}
+
+// R2C: the half spectra of a sequence's two real lines.
+template <typename R>
+__device__ __forceinline__ void rx_store_r2c(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
+  using Q = typename Vec<R>::Q;
+  using C = typename Cx<R>::T;
+  const PassArgs& A = X.p;
+  const int n = A.m, h = n / 2 + 1, lgG = X.g.lgG, total = h << lgG, P = X.g.P;
+  const unsigned mh = fdiv_magic(h);
+  C* out = reinterpret_cast<C*>(A.out);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    int g, k;
+    rx_item(it, lgG, h, mh, D.mode == 0, g, k);
+    const int l = g * 2 * Vec<R>::W;
+    if (l >= D.lines) continue;
+    const RxV<R> a = rows[k * P + g], b = rows[(k == 0 ? 0 : n - k) * P + g];
+    double f = A.scale * 0.5;
+    if (A.post_mode == W_HALF_INTERIOR && k != 0 && 2 * k != n) f *= A.post_factor;
+    const Q q = qc<Q>(f);
+    const Q xr = qmul(qadd(a.x, b.x), q), xi = qmul(qsub(a.y, b.y), q);
+    const Q yr = qmul(qadd(a.y, b.y), q), yi = qmul(qsub(b.x, a.x), q);
+    if constexpr (sizeof(R) == 4) {
+      const C v[4] = {make_float2(xr.v.x, xi.v.x), make_float2(yr.v.x, yi.v.x), make_float2(xr.v.y, xi.v.y),
+                      make_float2(yr.v.y, yi.v.y)};
+      if (D.mode == 0) {
+        C* o = out + D.at(k, l);
+        rx_put2(o, v[0], v[1], l + 1 < D.lines);
+        if (l + 2 < D.lines) rx_put2(o + 2, v[2], v[3], l + 3 < D.lines);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (l + j < D.lines) out[D.at(k, l + j)] = v[j];
+      }
+    } else {
+      out[D.at(k, l)] = make_double2(xr, xi);
+      if (l + 1 < D.lines) out[D.at(k, l + 1)] = make_double2(yr, yi);
+    }
+  }
+}
+
+// C2R: the real and imaginary parts are the two real lines.
+template <typename R>
+__device__ __forceinline__ void rx_store_c2r(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
+  const PassArgs& A = X.p;
+  const int n = A.m, lgG = X.g.lgG, total = n << lgG;
+  const unsigned mn = fdiv_magic(n);
+  const R sc = R(A.scale);
+  R* out = reinterpret_cast<R*>(A.out);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    int g, k;
+    rx_item(it, lgG, n, mn, D.mode == 0, g, k);
+    const int l = g * 2 * Vec<R>::W;
+    if (l >= D.lines) continue;
+    const RxV<R> z = rows[k * X.g.P + g];
+    R v[2 * Vec<R>::W];
+    if constexpr (sizeof(R) == 4) {
+      v[0] = z.x.v.x * sc;
+      v[1] = z.y.v.x * sc;
+      v[2] = z.x.v.y * sc;
+      v[3] = z.y.v.y * sc;
+    } else {
+      v[0] = z.x * sc;
+      v[1] = z.y * sc;
+    }
+    constexpr int NV = 2 * Vec<R>::W;
+    if (D.mode == 0) {
+      R* o = out + D.at(k, l);
+      if (l + NV <= D.lines && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+        if constexpr (sizeof(R) == 4)
+          *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+          *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+          if (l + j < D.lines) o[j] = v[j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if (l + j < D.lines) out[D.at(k, l + j)] = v[j];
+    }
+  }
+}
+
+// ---- real-to-real kinds: scalar access to the rows (sequence s, element q)
+template <typename R>
+__device__ __forceinline__ R* rx_slot(RxV<R>* rows, int P, int s, int q) {
+  if constexpr (sizeof(R) == 4)
+    return reinterpret_cast<R*>(rows + q * P + (s >> 1)) + (s & 1);
+  else
+    return reinterpret_cast<R*>(rows + q * P + s);
+}
+template <typename R>
+__device__ __forceinline__ typename Cx<R>::T rx_get(const RxV<R>* rows, int P, int s, int q) {
+  const R* p = rx_slot<R>(const_cast<RxV<R>*>(rows), P, s, q);
+  return mk<typename Cx<R>::T, R>(p[0], p[Vec<R>::W]);
+}
+
+// FFT input rows of a real-to-real pass from the staged lines (the
+// definitions of the generic kernel): Makhoul's reordering and pre-twiddle for
+// kinds II / III, the half-length (odd n: zero-padded) form of kinds IV, the
+// symmetric extensions of kinds I.  Sequence s is pair s (two real lines, or
+// the parts of a complex line); kinds IV take one sequence per line or part.
+template <typename R, int SUB>
+__device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows, const RxArgs& X, int lines) {
+  using C = typename Cx<R>::T;
+  const PassArgs& A = X.p;
+  const int n = A.n, m = A.m, P = X.g.P;
+  const int lgs = X.g.lgG + (sizeof(R) == 4 ? 1 : 0), total = m << lgs;
+  const R pre_f = R(A.pre_factor);
+  const C* aux0 = reinterpret_cast<const C*>(A.aux0);
+  const bool cplx = A.in_complex != 0;
+  const R zero = R(0);
+  auto getv = [&](int p, int c, int q) -> R {
+    R v;
+    if (cplx) {
+      v = p < lines ? reinterpret_cast<const R*>(S)[2 * (p * X.g.sl + q * X.g.sq) + c] : zero;
+    } else {
+      const int l = 2 * p + c;
+      v = l < lines ? reinterpret_cast<const R*>(S)[l * X.g.sl + q * X.g.sq] : zero;
+    }
+    if (A.pre_mode != W_NONE && weight_hit(A.pre_mode, q, n)) v *= pre_f;
+    return v;
+  };
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    const int s = it & ((1 << lgs) - 1), q = it >> lgs;
+    C z;
+    if constexpr (SUB == S_DCT2 || SUB == S_DST2) {
+      const int idx = (2 * q < n) ? 2 * q : 2 * (n - 1 - q) + 1;
+      R x = getv(s, 0, idx), y = getv(s, 1, idx);
+      if (SUB == S_DST2 && (idx & 1)) {
+        x = -x;
+        y = -y;
+      }
+      z = mk<C, R>(x, y);
+    } else if constexpr (SUB == S_DCT3 || SUB == S_DST3) {
+      const int i0 = SUB == S_DST3 ? n - 1 - q : q;
+      const R ux = getv(s, 0, i0), uy = getv(s, 1, i0);
+      R vx = zero, vy = zero;
+      if (q > 0) {
+        const int i1 = SUB == S_DST3 ? q - 1 : n - q;
+        vx = getv(s, 0, i1);
+        vy = getv(s, 1, i1);
+      }
+      const C w = aux0[q];
+      const C Vx = cmul(w, mk<C, R>(ux, -vx));
+      const C Vy = cmul(w, mk<C, R>(uy, -vy));
+      z = mk<C, R>(Vx.x - Vy.y, Vx.y + Vy.x);
+    } else if constexpr (SUB == S_DCT4 || SUB == S_DST4) {
+      const int p = s >> 1, c = s & 1;
+      if ((n & 1) == 0) {
+        const int i0 = 2 * q, i1 = n - 1 - 2 * q;
+        const int j0 = SUB == S_DST4 ? n - 1 - i0 : i0, j1 = SUB == S_DST4 ? n - 1 - i1 : i1;
+        z = cmul(mk<C, R>(getv(p, c, j0), getv(p, c, j1)), aux0[q]);
+      } else if (q < n) {
+        z = scl(aux0[q], getv(p, c, SUB == S_DST4 ? n - 1 - q : q));
+      } else {
+        z = mk<C, R>(zero, zero);
+      }
+    } else if constexpr (SUB == S_DCT1) {
+      const int idx = q <= n - 1 ? q : m - q;
+      z = mk<C, R>(getv(s, 0, idx), getv(s, 1, idx));
+    } else if constexpr (SUB == S_DST1) {
+      if (q == 0 || q == n + 1)
+        z = mk<C, R>(zero, zero);
+      else if (q <= n)
+        z = mk<C, R>(getv(s, 0, q - 1), getv(s, 1, q - 1));
+      else
+        z = mk<C, R>(-getv(s, 0, m - q - 1), -getv(s, 1, m - q - 1));
+    } else {  // DHT
+      z = mk<C, R>(getv(s, 0, q), getv(s, 1, q));
+    }
+    R* o = rx_slot<R>(rows, P, s, (A.inv && q != 0) ? m - q : q);
+    o[0] = z.x;
+    o[Vec<R>::W] = z.y;
+  }
+}
+
+// Outputs of a real-to-real pass from the finished rows.
+template <typename R, int SUB>
+__device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
+  using C = typename Cx<R>::T;
+  const PassArgs& A = X.p;
+  const int n = A.n, P = X.g.P;
+  constexpr bool iv4 = SUB == S_DCT4 || SUB == S_DST4;
+  const int lgp = X.g.lgG + (sizeof(R) == 4 ? 1 : 0) - (iv4 ? 1 : 0);  // pairs per tile
+  const int total = n << lgp;
+  const unsigned mn = fdiv_magic(n);
+  const R post_f = R(A.post_factor), sc = R(A.scale), h = R(0.5);
+  const C* aux0 = reinterpret_cast<const C*>(A.aux0);
+  const C* aux1 = reinterpret_cast<const C*>(A.aux1);
+  for (int it = threadIdx.x; it < total; it += blockDim.x) {
+    int p, k;
+    rx_item(it, lgp, n, mn, D.mode == 0, p, k);
+    const int l = A.out_complex ? p : 2 * p;
+    if (l >= D.lines) continue;
+    R v0, v1;
+    if constexpr (SUB == S_DCT2 || SUB == S_DST2 || SUB == S_DHT) {
+      const int kk = SUB == S_DST2 ? n - 1 - k : k;
+      const C a = rx_get<R>(rows, P, p, kk), b = rx_get<R>(rows, P, p, kk == 0 ? 0 : n - kk);
+      const C V = mk<C, R>((a.x + b.x) * h, (a.y - b.y) * h), U = mk<C, R>((a.y + b.y) * h, (b.x - a.x) * h);
+      if constexpr (SUB == S_DHT) {
+        v0 = V.x - V.y;
+        v1 = U.x - U.y;
+      } else {
+        const C w = aux0[kk];
+        v0 = R(2) * (w.x * V.x - w.y * V.y);
+        v1 = R(2) * (w.x * U.x - w.y * U.y);
+      }
+    } else if constexpr (SUB == S_DCT3 || SUB == S_DST3) {
+      const C z = rx_get<R>(rows, P, p, (k & 1) ? n - 1 - (k >> 1) : (k >> 1));
+      const bool neg = SUB == S_DST3 && (k & 1);
+      v0 = neg ? -z.x : z.x;
+      v1 = neg ? -z.y : z.y;
+    } else if constexpr (iv4) {
+      auto one = [&](int s) -> R {
+        R v;
+        if ((n & 1) == 0) {
+          if ((k & 1) == 0)
+            v = R(2) * cmul(rx_get<R>(rows, P, s, k >> 1), aux1[k >> 1]).x;
+          else
+            v = R(-2) * cmul(rx_get<R>(rows, P, s, (n - 1 - k) >> 1), aux1[(n - 1 - k) >> 1]).y;
+        } else {
+          v = R(2) * cmul(rx_get<R>(rows, P, s, k), aux1[k]).x;
+        }
+        return (SUB == S_DST4 && (k & 1)) ? -v : v;
+      };
+      v0 = one(2 * p);
+      v1 = one(2 * p + 1);
+    } else if constexpr (SUB == S_DCT1) {
+      const C z = rx_get<R>(rows, P, p, k);
+      v0 = z.x;
+      v1 = z.y;
+    } else {  // DST-I
+      const C z = rx_get<R>(rows, P, p, k + 1);
+      v0 = -z.y;
+      v1 = z.x;
+    }
+    R f = sc;
+    if (A.post_mode != W_NONE && weight_hit(A.post_mode, k, n)) f *= post_f;
+    v0 *= f;
+    v1 *= f;
+    if (A.out_complex) {
+      reinterpret_cast<C*>(A.out)[D.at(k, l)] = mk<C, R>(v0, v1);
+    } else {
+      R* out = reinterpret_cast<R*>(A.out);
+      const long long o = D.at(k, l);
+      if (l + 1 >= D.lines) {
+        out[o] = v0;
+      } else if (D.mode == 0 && (reinterpret_cast<uintptr_t>(out + o) & (2 * sizeof(R) - 1)) == 0) {
+        *reinterpret_cast<C*>(out + o) = mk<C, R>(v0, v1);
+      } else {
+        out[o] = v0;
+        out[D.at(k, l + 1)] = v1;
+      }
+    }
+  }
+}
+
+#define RX_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+#define RX_SUBS(X) \
+  X(S_DCT1) X(S_DCT2) X(S_DCT3) X(S_DCT4) X(S_DST1) X(S_DST2) X(S_DST3) X(S_DST4) X(S_DHT)
+
+// TR: the pass stores transposed (C2C only; the other kinds choose at run time).
+template <typename R, int KIND, bool TR>
+__global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_constant__ RxArgs X) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using V = RxV<R>;
+  const PassArgs& A = X.p;
+  const RxGeom& g = X.g;
+  if (A.gate != nullptr && *A.gate != 0) return;
+  long long tile = blockIdx.x;
+  const long long step = gridDim.x, end = A.ntiles;
+  if (tile >= end) return;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  V* b0 = reinterpret_cast<V*>(smem);
+  V* b1 = b0 + g.bufv;
+  V* W = reinterpret_cast<V*>(smem + g.off_tw);
+  unsigned char* S = smem + g.off_stage;
+  TileAddr* desc = reinterpret_cast<TileAddr*>(smem + g.off_desc);     // tiles i, i+1, i+2
+  PieceAddr* prow = reinterpret_cast<PieceAddr*>(desc + 3);            // pieces of tiles i, i+1
+  const V* Wg = reinterpret_cast<const V*>(A.twiddle);
+  const V* tw = g.tw_smem ? W : Wg;
+  const TileAddr* tiles = reinterpret_cast<const TileAddr*>(A.tile_tab);
+  const PieceAddr* pieces = reinterpret_cast<const PieceAddr*>(A.piece_tab);
+  const int mode = KIND == P_C2C && TR ? 0 : A.dst_k_contig;
+  const int np = mode == 1 ? 0 : A.npieces;
+  RxDst D;
+  D.mode = mode;
+  D.np = np;
+  D.nout = A.n_out;
+  D.mnout = fdiv_magic(A.n_out);
+  // this thread's piece starts at output index pst
+  const long long pst = np > 0 ? (long long)A.n_out * tid / np : 0;
+
+  if (tid == 0) {
+    desc[0] = load_tile(tiles, tile);
+    if (tile + step < end) desc[1] = load_tile(tiles, tile + step);
+  }
+  if (tid < np) prow[tid] = pieces[tile * np + tid];
+  for (int i = tid; i < g.tw_smem; i += nt) W[i] = Wg[i];
+  __syncthreads();
+  rx_stage<R, KIND>(S, X, desc[0]);
+  rx_cp_commit();
+
+  int par = 0;
+  for (int i = 0;; i = i == 2 ? 0 : i + 1, tile += step, par ^= kRxMaxPieces) {
+    rx_cp_wait();
+    PieceAddr* pr = prow + par;
+    PieceAddr* pr_next = prow + (par ^ kRxMaxPieces);
+    if (tid < np) {
+      PieceAddr pa = pr[tid];
+      pa.rowbase -= mode == 0 ? pst * pa.stride : pst;
+      pr[tid] = pa;
+    }
+    __syncthreads();  // staged lines, descriptors and pieces in place; the previous tile's rows are free
+    const TileAddr& ta = desc[i];
+    const TileAddr& tn = desc[i == 2 ? 0 : i + 1];
+    D.dst0 = ta.dst0;
+    D.dstb = ta.dstb;
+    D.lines = ta.lines;
+    D.prow = pr;
+
+    int s0 = 1, NS = 1;
+    if constexpr (KIND == P_R2R) {
+      s0 = 0;
+      switch (A.sub) {
+#define X_(u) \
+  case u: rx_pre_r2r<R, u>(S, b0, X, ta.lines); break;
+        RX_SUBS(X_)
+#undef X_
+      }
+    } else {
+      if (g.pre) {
+        s0 = 0;
+        rx_rows<R, KIND>(S, b0, X);
+      } else {
+        NS = A.radix[0];
+        switch (A.radix[0]) {
+#define X_(r) \
+  case r: rx_first<R, KIND, r>(S, b0, X); break;
+          RX_RADICES(X_)
+#undef X_
+        }
+      }
+    }
+    __syncthreads();
+    const bool has_next = tile + step < end;
+    if (has_next) {
+      if (!g.alias) rx_stage<R, KIND>(S, X, tn);
+      if (tid == 0 && tile + 2 * step < end) {
+        TileAddr* d = desc + (i == 0 ? 2 : i - 1);
+        const TileAddr* t = tiles + tile + 2 * step;
+        rx_cp_async<16>(d, t);
+        rx_cp_async<16>(reinterpret_cast<char*>(d) + 16, reinterpret_cast<const char*>(t) + 16);
+      }
+      if (tid < np) rx_cp_async<16>(pr_next + tid, pieces + (tile + step) * np + tid);
+      rx_cp_commit();
+    }
+    V *in = b0, *out = b1;
+    // a C2C pass ends with the stage that stores; the others finish the rows
+    const bool fused = KIND == P_C2C && A.nstages > s0 && A.radix[A.nstages - 1] <= kRxRegRadix && A.nstages > 1;
+    const int last = fused ? A.nstages - 1 : A.nstages;
+    for (int s = s0; s < last; ++s) {
+      const int rad = A.radix[s];
+      const V* t = tw + g.twoff[s];
+      switch (rad) {
+#define X_(r) \
+  case r: rx_mid<R, r>(in, out, X, NS, t); break;
+        RX_RADICES(X_)
+#undef X_
+        default: rx_mid_prime<R>(in, out, X, rad, NS, t, t + (s > 0 ? (rad - 1) * NS : 0)); break;
+      }
+      __syncthreads();
+      NS *= rad;
+      V* u = in;
+      in = out;
+      out = u;
+    }
+    if constexpr (KIND == P_C2C) {
+      if (fused) {
+        const V* t = tw + g.twoff[last];
+        switch (A.radix[last]) {
+#define X_(r) \
+  case r: rx_last<R, r, TR>(in, X, t, D); break;
+          RX_RADICES(X_)
+#undef X_
+        }
+      } else {
+        rx_store_c2c<R>(in, X, D);
+      }
+    } else if constexpr (KIND == P_R2C) {
+      rx_store_r2c<R>(in, X, D);
+    } else if constexpr (KIND == P_C2R) {
+      rx_store_c2r<R>(in, X, D);
+    } else {
+      switch (A.sub) {
+#define X_(u) \
+  case u: rx_post_r2r<R, u>(in, X, D); break;
+        RX_SUBS(X_)
+#undef X_
+      }
+    }
+    if (!has_next) break;
+    if (g.alias) {
+      __syncthreads();  // the staging area is the second row buffer
+      rx_stage<R, KIND>(S, X, tn);
+      rx_cp_commit();
+    }
+  }
+}
+
+}  // namespace pb

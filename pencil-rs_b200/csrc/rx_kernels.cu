@@ -1,0 +1,42 @@
+// Instantiations and launchers of the runtime-radix pass kernel, one object
+// per kind (RX_KIND: 1 C2C, 2 R2C, 3 C2R, 4 real-to-real).
+#include "rx_kernel.cuh"
+
+namespace pb {
+
+template <int KIND>
+using RxFn = void (*)(const RxArgs);
+
+template <typename R>
+static RxFn<RX_KIND> rx_pick(const PassArgs& A) {
+  if constexpr (RX_KIND == P_C2C)
+    return A.dst_k_contig == 0 ? rx_kernel<R, RX_KIND, true> : rx_kernel<R, RX_KIND, false>;
+  else
+    return rx_kernel<R, RX_KIND, false>;
+}
+
+template <int KIND>
+cudaError_t rx_launch_kind(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream);
+template <int KIND>
+int rx_occupancy_kind(const RxArgs& X, int real_bytes);
+
+template <>
+cudaError_t rx_launch_kind<RX_KIND>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream) {
+  const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem);
+  if (err != cudaSuccess) return err;
+  kern<<<dim3((unsigned)grid), X.g.threads, X.g.smem, stream>>>(X);
+  return cudaGetLastError();
+}
+
+template <>
+int rx_occupancy_kind<RX_KIND>(const RxArgs& X, int real_bytes) {
+  const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
+  int blocks = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, X.g.threads, X.g.smem) != cudaSuccess)
+    return 1;
+  return blocks > 0 ? blocks : 1;
+}
+
+}  // namespace pb

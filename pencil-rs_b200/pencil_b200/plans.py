@@ -318,12 +318,13 @@ class _Plan:
         """Kernel family of each launch of one operation: "generic", "check",
         "pow2" (register-resident power-of-two pass), "mixed_radix" or
         "bluestein" (a C2C / R2C / C2R length with a prime factor above 31 on
-        the mixed-radix kernel)."""
+        the mixed-radix kernel) or "runtime_radix" (other lengths with prime
+        factors up to 31)."""
         cap = 64
         ks = (C.c_int32 * cap)()
         cnt = C.c_int32()
         L.check(L.load().pb_plan_step_kernels(self._h, op, ks, cap, C.byref(cnt)), "step kernels")
-        names = ("generic", "check", "pow2", "mixed_radix", "bluestein")
+        names = ("generic", "check", "pow2", "mixed_radix", "bluestein", "runtime_radix")
         return [names[ks[i]] for i in range(cnt.value)]
 
     # in-place single-allocation arrays (C2cInPlaceArray / R2cInPlaceArray)
@@ -373,7 +374,7 @@ class _Plan:
         """Per launch of `op`: kernel family, FFT length, lines per tile,
         persistent grid, CTAs per SM, schedule, radices and whether the
         autotuner chose it."""
-        names = ("generic", "check", "pow2", "mixed_radix", "bluestein")
+        names = ("generic", "check", "pow2", "mixed_radix", "bluestein", "runtime_radix")
         out = []
         for i in range(len(self.step_kinds(op))):
             c = L.PbStepConfig()
