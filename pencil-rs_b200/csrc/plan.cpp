@@ -706,10 +706,10 @@ static std::vector<int> radices(int m) {
   return r;
 }
 
-// Bluestein: the convolution length (a power of two >= 2m - 1) when m has a
-// prime factor above 31 -- where the generic kernel's O(p) radix costs more
-// per point than two power-of-two FFTs of about 2-4 m points -- and the three
-// M-point buffers fit shared memory (M <= 4096 f32, 2048 f64); else 0.
+// Bluestein: the convolution length (7-smooth, >= 2m - 1) when m has a prime
+// factor above 31 -- where an O(p) radix costs more per point than two FFTs of
+// about 2-2.5 m points -- and the generic kernel's three M-point buffers fit
+// shared memory (M <= 4096 f32, 2048 f64); else 0.
 static int bluestein_len(int m, int real_bytes) {
   int r = m, big = 1;
   for (int p = 2; (long long)p * p <= r; ++p)
@@ -721,9 +721,10 @@ static int bluestein_len(int m, int real_bytes) {
   if (big <= 31) return 0;
   for (int L : kBluesteinLengths)
     if (L >= 2 * m - 1) return L;
-  int M = 1;
-  while (M < 2 * m - 1) M <<= 1;
-  return M <= (real_bytes == 4 ? 4096 : 2048) ? M : 0;
+  // longer ones: lengths with three stages of radices up to 16
+  for (int L : {1152, 1280, 1536, 1792, 2048, 2304, 2560, 3072, 3584, 4096})
+    if (L >= 2 * m - 1) return L <= (real_bytes == 4 ? 4096 : 2048) ? L : 0;
+  return 0;
 }
 
 // The chirp w_j = exp(-i pi j^2 / m) of a forward pass (conjugated for an
@@ -752,10 +753,37 @@ static size_t chirp_table(pb_plan& P, int m, int inv) {
   return off;
 }
 
+// The n-point DFT (negative exponent) of x[0], x[st], ... in long double:
+// decimation by the smallest factor; n * st = M, (cs, sn) the M-th roots.
+static void host_dft(int M, int n, int st, const long double* xr, const long double* xi, long double* yr,
+                     long double* yi, const std::vector<long double>& cs, const std::vector<long double>& sn) {
+  if (n == 1) {
+    yr[0] = xr[0];
+    yi[0] = xi[0];
+    return;
+  }
+  int p = 2;
+  while (n % p) ++p;
+  const int h = n / p;
+  std::vector<long double> ar(n), ai(n);
+  for (int j = 0; j < p; ++j)
+    host_dft(M, h, st * p, xr + (size_t)j * st, xi + (size_t)j * st, &ar[(size_t)j * h], &ai[(size_t)j * h], cs, sn);
+  for (int k = 0; k < n; ++k) {
+    long double sr = 0.0L, si = 0.0L;
+    for (int j = 0; j < p; ++j) {
+      const int q = (int)((long long)j * k % n) * st;  // exp(-2 pi i j k / n)
+      const long double a = ar[(size_t)j * h + k % h], b = ai[(size_t)j * h + k % h];
+      sr += a * cs[q] + b * sn[q];
+      si += b * cs[q] - a * sn[q];
+    }
+    yr[k] = sr;
+    yi[k] = si;
+  }
+}
+
 // The DFT (negative exponent) of the M-periodic conjugate chirp b_j =
 // conj(w_j), b_{M-j} = b_j (0 < j < m), zero elsewhere, divided by M: the
-// convolution's kernel.  In long double, rounded once: a radix-2 FFT for
-// powers of two, else the direct sum with exact angle indices (j k mod M).
+// convolution's kernel.  In long double, rounded once.
 static size_t bluestein_kernel_table(pb_plan& P, int m, int M, int inv) {
   const std::string key =
       "BK" + std::to_string(m) + "_" + std::to_string(M) + "i" + std::to_string(inv) + "r" + std::to_string(P.real_bytes);
@@ -773,53 +801,14 @@ static size_t bluestein_kernel_table(pb_plan& P, int m, int M, int inv) {
       im[M - j] = im[j];
     }
   }
-  if (M & (M - 1)) {
-    std::vector<long double> cs(M), sn(M);
-    for (int q = 0; q < M; ++q) {
-      cs[q] = cosl(2.0L * pi * (long double)q / (long double)M);
-      sn[q] = sinl(2.0L * pi * (long double)q / (long double)M);
-    }
-    std::vector<long double> fr(M, 0.0L), fi(M, 0.0L);
-    for (int k = 0; k < M; ++k) {
-      long double ar = 0.0L, ai = 0.0L;
-      int q = 0;  // j k mod M
-      for (int j = 0; j < M; ++j) {
-        // (re + i im) * exp(-2 pi i q / M)
-        ar += re[j] * cs[q] + im[j] * sn[q];
-        ai += im[j] * cs[q] - re[j] * sn[q];
-        q += k;
-        if (q >= M) q -= M;
-      }
-      fr[k] = ar;
-      fi[k] = ai;
-    }
-    re.swap(fr);
-    im.swap(fi);
-  } else {
-  // bit-reversal permutation, then iterative butterflies
-  for (int i = 1, j = 0; i < M; ++i) {
-    int bit = M >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) {
-      std::swap(re[i], re[j]);
-      std::swap(im[i], im[j]);
-    }
+  std::vector<long double> cs(M), sn(M), fr(M), fi(M);
+  for (int q = 0; q < M; ++q) {
+    cs[q] = cosl(2.0L * pi * (long double)q / (long double)M);
+    sn[q] = sinl(2.0L * pi * (long double)q / (long double)M);
   }
-  for (int len = 2; len <= M; len <<= 1) {
-    for (int i = 0; i < M; i += len)
-      for (int k = 0; k < len / 2; ++k) {
-        const long double th = -2.0L * pi * (long double)k / (long double)len;
-        const long double c = cosl(th), sn = sinl(th);
-        const int a = i + k, b = i + k + len / 2;
-        const long double xr = re[b] * c - im[b] * sn, xi = re[b] * sn + im[b] * c;
-        re[b] = re[a] - xr;
-        im[b] = im[a] - xi;
-        re[a] += xr;
-        im[a] += xi;
-      }
-  }
-  }
+  host_dft(M, M, 1, re.data(), im.data(), fr.data(), fi.data(), cs, sn);
+  re.swap(fr);
+  im.swap(fi);
   std::vector<double> d(2 * (size_t)M);
   for (int k = 0; k < M; ++k) {
     d[2 * k] = (double)(re[k] / (long double)M);
@@ -1051,7 +1040,7 @@ static size_t rx_table(pb_plan& P, const PassArgs& A) {
   for (int r : rad) key += "_" + std::to_string(r);
   auto it = P.cache.find(key);
   if (it != P.cache.end()) return it->second;
-  const size_t roots = roots_table(P, A.m);
+  const size_t roots = roots_table(P, A.bs_m2 ? A.bs_m2 : A.m);
   size_t off;
   if (P.real_bytes == 4) {
     const std::vector<float> t = rx_twiddles<float>(rad, reinterpret_cast<const float*>(&P.host.bytes[roots]));
@@ -1060,6 +1049,20 @@ static size_t rx_table(pb_plan& P, const PassArgs& A) {
     const std::vector<double> t = rx_twiddles<double>(rad, reinterpret_cast<const double*>(&P.host.bytes[roots]));
     off = P.host.add(t.data(), t.size() * sizeof(double));
   }
+  P.cache[key] = off;
+  return off;
+}
+
+// A table of n complex values as the runtime-radix kernel's vectors.
+static size_t rx_vectors(pb_plan& P, size_t table, int n) {
+  if (P.real_bytes == 8) return table;
+  const std::string key = "V" + std::to_string(table);
+  auto it = P.cache.find(key);
+  if (it != P.cache.end()) return it->second;
+  const float* t = reinterpret_cast<const float*>(&P.host.bytes[table]);
+  std::vector<float> v;
+  for (int i = 0; i < 2 * n; ++i) v.insert(v.end(), 2, t[i]);
+  const size_t off = P.host.add(v.data(), v.size() * sizeof(float));
   P.cache[key] = off;
   return off;
 }
@@ -1371,10 +1374,10 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
       A.lines = L;
     }
   }
-  // every other length with prime factors up to 31, any kind: the
-  // runtime-radix kernel, on the same layouts (the split direct store for
-  // every kind)
-  if (!A.fast && !P.force_generic && op.kind != P_COPY && !A.bs_m2 && (src.perm[N - 1] == a || r2r_strided) &&
+  // every other length and kind: the runtime-radix kernel (Bluestein's form
+  // above 31 included), on the same layouts (the split direct store for every
+  // kind)
+  if (!A.fast && !P.force_generic && op.kind != P_COPY && (src.perm[N - 1] == a || r2r_strided) &&
       src.split_of(a) < 0) {
     const int ta = dst.split_of(a);
     const bool direct = dst.perm[N - 1] == a && ta < 0;
@@ -1391,6 +1394,10 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
         A = B;
         A.fast = 5;
         A.twiddle = enc(rx_table(P, A));
+        if (A.bs_m2) {
+          A.bs_chirp = enc(rx_vectors(P, chirp_table(P, A.m, A.inv), A.m));
+          A.bs_kernel = enc(rx_vectors(P, bluestein_kernel_table(P, A.m, A.bs_m2, A.inv), A.bs_m2));
+        }
         L = A.lines;
       }
     }
@@ -2256,7 +2263,7 @@ int pb_plan_step_kernels(const pb_plan* plan, int32_t op, int32_t* kernels, int3
     const Program& prog = plan->prog[user_mode(*plan, op)];
     int n = 0;
     for (const Step& s : prog.steps) {
-      const int k = s.type != 0 ? 1 : (s.pa.fast == 1 ? 2 : (s.pa.fast >= 4 ? s.pa.fast : (s.pa.fast >= 2 ? 3 : 0)));
+      const int k = s.type != 0 ? 1 : (s.pa.fast == 1 ? 2 : (s.pa.fast >= 4 ? (s.pa.bs_m2 ? 4 : 5) : (s.pa.fast >= 2 ? 3 : 0)));
       if (kernels && n < capacity) kernels[n] = k;
       ++n;
     }
@@ -4550,7 +4557,7 @@ int pb_plan_step_config(const pb_plan* plan, int32_t op, int32_t step, pb_step_c
     }
     const PassArgs& A = st.pa;
     const int sms = sm_count();
-    out->kernel = A.fast == 1 ? 2 : (A.fast == 2 || A.fast == 3) ? 3 : (A.fast >= 4 ? A.fast : 0);
+    out->kernel = A.fast == 1 ? 2 : (A.fast == 2 || A.fast == 3) ? 3 : (A.fast >= 4 ? (A.bs_m2 ? 4 : 5) : 0);
     out->fft_len = A.m;
     out->lines = A.lines;
     out->grid_ctas = A.fast ? (int)std::min<long long>(A.grid_ctas, A.ntiles) : 0;
@@ -4567,7 +4574,11 @@ int pb_plan_step_config(const pb_plan* plan, int32_t op, int32_t step, pb_step_c
     else if (A.fast == 1)
       out->nradix = pow2_radices(A.m, out->radix, 12);
 
-    else {
+    else if (A.bs_m2) {  // the convolution length, as its prime-power factors
+      const std::vector<int> r = radices(A.bs_m2);
+      out->nradix = std::min((int)r.size(), 12);
+      for (int i = 0; i < out->nradix; ++i) out->radix[i] = r[i];
+    } else {
       out->nradix = std::min(A.nstages, 12);
       for (int i = 0; i < out->nradix; ++i) out->radix[i] = A.radix[i];
     }

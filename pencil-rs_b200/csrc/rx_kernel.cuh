@@ -1,6 +1,12 @@
 // Fused pass with stage radices chosen at run time, for the lengths that have
 // no compiled kernel of their own: C2C, R2C, C2R and the real-to-real kinds on
-// any length whose prime factors are at most 31.
+// any length whose prime factors are at most 31, and (BS) Bluestein's chirp-z
+// form of the others: two transforms of the convolution length without leaving
+// shared memory, the chirp and the kernel multiplied in as their first stages
+// read the rows.  Bluestein passes of the generic kernel ran at 0.06-0.17 TB/s
+// (DST-I 100 and 256, DCT-I 384); here 0.23-0.37, and 0.46-0.8 on DCT-II 257
+// and DCT-IV 94.  C2C, R2C and C2R convolutions up to 1024 points keep the
+// compiled kernel (mr_bs.cuh), which is 1.1-1.7 times faster than this one.
 //
 // Persistent CTAs walk the pass's tiles.  The lines of the next tile are
 // copied to a staging area by cp.async while the current tile is transformed,
@@ -146,12 +152,12 @@ __device__ __forceinline__ RxV<R> rx_fetch_at(const unsigned char* S, int base, 
 
 // C2R: Hermitian extension X + iY of the half spectra of lines 2s and 2s + 1
 // at element q of the (index-reversed for a positive exponent) sequence.
-template <typename R>
+template <typename R, bool BS>
 __device__ __forceinline__ RxV<R> rx_fetch_c2r(const unsigned char* S, const RxArgs& X, int g, int q) {
   using C = typename Cx<R>::T;
   const PassArgs& A = X.p;
   const int m = A.m;
-  if (A.inv && q != 0) q = m - q;
+  if (!BS && A.inv && q != 0) q = m - q;
   const bool mirror = 2 * q > m;
   const int hq = mirror ? m - q : q;
   const bool edge = hq == 0 || 2 * hq == m;
@@ -195,7 +201,7 @@ __device__ __forceinline__ void rx_first(const unsigned char* S, RxV<R>* out, co
     RxV<R> v[RAD];
     if constexpr (KIND == P_C2R) {
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) v[r] = rx_fetch_c2r<R>(S, X, g, jb + r * NB);
+      for (int r = 0; r < RAD; ++r) v[r] = rx_fetch_c2r<R, false>(S, X, g, jb + r * NB);
     } else {
       // element jb + r*NB, or m - jb - r*NB (0 for element 0) when inverse
       const int base = g * rx_lines_per_vec<R, KIND>() * sl;
@@ -212,46 +218,76 @@ __device__ __forceinline__ void rx_first(const unsigned char* S, RxV<R>* out, co
 }
 
 // Rows from the staged lines without a stage (lengths whose stage 0 is a
-// direct-sum prime).
-template <typename R, int KIND>
+// direct-sum prime, and Bluestein passes, whose chirp carries the sign).
+template <typename R, int KIND, bool BS>
 __device__ __forceinline__ void rx_rows(const unsigned char* S, RxV<R>* out, const RxArgs& X) {
   const PassArgs& A = X.p;
   const int m = A.m, lgG = X.g.lgG, P = X.g.P, total = m << lgG;
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
     const int g = it & ((1 << lgG) - 1), q = it >> lgG;
     if constexpr (KIND == P_C2R) {
-      out[q * P + g] = rx_fetch_c2r<R>(S, X, g, q);
+      out[q * P + g] = rx_fetch_c2r<R, BS>(S, X, g, q);
     } else {
-      const int e = (A.inv && q != 0) ? m - q : q;
+      const int e = (!BS && A.inv && q != 0) ? m - q : q;
       out[q * P + g] = rx_fetch_at<R, KIND>(S, g * rx_lines_per_vec<R, KIND>() * X.g.sl, X.g.sl, e * X.g.sq);
     }
   }
 }
 
-// Stockham stage: butterfly jb (k = jb mod NS) takes rows jb + r*m/RAD times
-// W^{k r} and writes rows (jb - k)*RAD + k + r*NS.
-template <typename R, int RAD>
-__device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int NS, const RxV<R>* tw) {
+// Stockham stage: butterfly jb (k = jb mod NS) takes rows jb + r*len/RAD times
+// W^{k r} and writes rows (jb - k)*RAD + k + r*NS.  The first stage of each of
+// a Bluestein pass's two transforms (kMidMul, NS = 1) multiplies row i by
+// vector i of `mul` (the chirp, rows from `lim` on are zero; the convolution
+// kernel); its very last stage (kMidOut) reads the inverse transform off in
+// reversed order, row i being output len - i, and multiplies the outputs
+// below `lim` by the chirp.
+enum { kMidPlain = 0, kMidMul = 1, kMidOut = 2 };
+template <typename Q>
+__device__ __forceinline__ VC<Q> rx_ldg(const VC<Q>* p) {
+  const float4 f = __ldg(reinterpret_cast<const float4*>(p));
+  VC<Q> r;
+  *reinterpret_cast<float4*>(&r) = f;
+  return r;
+}
+template <typename R, int RAD, int MODE>
+__device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int NS, const RxV<R>* tw,
+                                       const RxV<R>* mul, int lim) {
   using Q = typename Vec<R>::Q;
-  const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
+  const int len = X.g.len, NB = len / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
   const int rs = NB * P, ws = NS * P;
   const unsigned mNS = fdiv_magic(NS);
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
     const int g = it & ((1 << lgG) - 1), jb = it >> lgG;
-    const int k = jb - (int)fdiv(jb, NS, mNS) * NS;
+    const int k = MODE == kMidMul ? 0 : jb - (int)fdiv(jb, NS, mNS) * NS;
     const RxV<R>* p = in + jb * P + g;
     RxV<R> v[RAD];
+    if constexpr (MODE == kMidMul) {
 #pragma unroll
-    for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
-    if (NS > 1) {
-      const RxV<R>* t = tw + k;
+      for (int r = 0; r < RAD; ++r) {
+        const int i = jb + r * NB;
+        v[r] = i < lim ? vtw(p[r * rs], rx_ldg(mul + i)) : RxV<R>{qc<Q>(0.0), qc<Q>(0.0)};
+      }
+    } else {
 #pragma unroll
-      for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NS]);
+      for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
+      if (NS > 1) {
+        const RxV<R>* t = tw + k;
+#pragma unroll
+        for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NS]);
+      }
     }
     VB<Q, RAD>::run(v);
-    RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
+    if constexpr (MODE == kMidOut) {
 #pragma unroll
-    for (int r = 0; r < RAD; ++r) o[r * ws] = v[r];
+      for (int r = 0; r < RAD; ++r) {
+        const int i = (jb - k) * RAD + k + r * NS, o = i == 0 ? 0 : len - i;
+        if (o < lim) out[o * P + g] = vtw(v[r], rx_ldg(mul + o));
+      }
+    } else {
+      RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
+#pragma unroll
+      for (int r = 0; r < RAD; ++r) o[r * ws] = v[r];
+    }
   }
 }
 
@@ -261,7 +297,7 @@ __device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxAr
 template <typename R>
 __device__ __forceinline__ void rx_mid_prime(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int RAD, int NS,
                                              const RxV<R>* tw, const RxV<R>* roots) {
-  const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P;
+  const int NB = X.g.len / RAD, lgG = X.g.lgG, P = X.g.P;
   const int H = (RAD - 1) / 2, total = (NB * (H + 1)) << lgG;
   const int rs = NB * P, ws = NS * P;
   const unsigned mNS = fdiv_magic(NS), mNB = fdiv_magic(NB);
@@ -528,7 +564,7 @@ __device__ __forceinline__ typename Cx<R>::T rx_get(const RxV<R>* rows, int P, i
 // kinds II / III, the half-length (odd n: zero-padded) form of kinds IV, the
 // symmetric extensions of kinds I.  Sequence s is pair s (two real lines, or
 // the parts of a complex line); kinds IV take one sequence per line or part.
-template <typename R, int SUB>
+template <typename R, int SUB, bool BS>
 __device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows, const RxArgs& X, int lines) {
   using C = typename Cx<R>::T;
   const PassArgs& A = X.p;
@@ -597,7 +633,7 @@ __device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows,
     } else {  // DHT
       z = mk<C, R>(getv(s, 0, q), getv(s, 1, q));
     }
-    R* o = rx_slot<R>(rows, P, s, (A.inv && q != 0) ? m - q : q);
+    R* o = rx_slot<R>(rows, P, s, (!BS && A.inv && q != 0) ? m - q : q);
     o[0] = z.x;
     o[Vec<R>::W] = z.y;
   }
@@ -688,8 +724,9 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
 #define RX_SUBS(X) \
   X(S_DCT1) X(S_DCT2) X(S_DCT3) X(S_DCT4) X(S_DST1) X(S_DST2) X(S_DST3) X(S_DST4) X(S_DHT)
 
-// TR: the pass stores transposed (C2C only; the other kinds choose at run time).
-template <typename R, int KIND, bool TR>
+// TR: the pass stores transposed (C2C only; the other kinds choose at run
+// time).  BS: the m-point transform as a Bluestein convolution of length g.len.
+template <typename R, int KIND, bool TR, bool BS>
 __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_constant__ RxArgs X) {
   extern __shared__ __align__(16) unsigned char smem[];
   using V = RxV<R>;
@@ -753,15 +790,15 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
       s0 = 0;
       switch (A.sub) {
 #define X_(u) \
-  case u: rx_pre_r2r<R, u>(S, b0, X, ta.lines); break;
+  case u: rx_pre_r2r<R, u, BS>(S, b0, X, ta.lines); break;
         RX_SUBS(X_)
 #undef X_
       }
     } else {
-      if (g.pre) {
+      if (BS || g.pre) {
         s0 = 0;
-        rx_rows<R, KIND>(S, b0, X);
-      } else {
+        rx_rows<R, KIND, BS>(S, b0, X);
+      } else if constexpr (!BS) {
         NS = A.radix[0];
         switch (A.radix[0]) {
 #define X_(r) \
@@ -786,25 +823,69 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
     }
     V *in = b0, *out = b1;
     // a C2C pass ends with the stage that stores; the others finish the rows
-    const bool fused = KIND == P_C2C && A.nstages > s0 && A.radix[A.nstages - 1] <= kRxRegRadix && A.nstages > 1;
+    const bool fused =
+        !BS && KIND == P_C2C && A.nstages > s0 && A.radix[A.nstages - 1] <= kRxRegRadix && A.nstages > 1;
     const int last = fused ? A.nstages - 1 : A.nstages;
-    for (int s = s0; s < last; ++s) {
-      const int rad = A.radix[s];
-      const V* t = tw + g.twoff[s];
-      switch (rad) {
-#define X_(r) \
-  case r: rx_mid<R, r>(in, out, X, NS, t); break;
-        RX_RADICES(X_)
-#undef X_
-        default: rx_mid_prime<R>(in, out, X, rad, NS, t, t + (s > 0 ? (rad - 1) * NS : 0)); break;
-      }
+    auto swap = [&] {
       __syncthreads();
-      NS *= rad;
       V* u = in;
       in = out;
       out = u;
+    };
+    if constexpr (BS) {
+      const V* chirp = reinterpret_cast<const V*>(A.bs_chirp);
+      const V* ker = reinterpret_cast<const V*>(A.bs_kernel);
+      for (int f = 0; f < 2; ++f) {
+        const V* mul = f ? ker : chirp;
+        const int lim = f ? g.len : A.m;
+        switch (A.radix[0]) {
+#define X_(r) \
+  case r: rx_mid<R, r, kMidMul>(in, out, X, 1, nullptr, mul, lim); break;
+          RX_RADICES(X_)
+#undef X_
+        }
+        swap();
+        NS = A.radix[0];
+        for (int s = 1; s < A.nstages; ++s) {
+          const int rad = A.radix[s];
+          const V* t = tw + g.twoff[s];
+          if (f == 1 && s == A.nstages - 1) {
+            switch (rad) {
+#define X_(r) \
+  case r: rx_mid<R, r, kMidOut>(in, out, X, NS, t, chirp, A.m); break;
+              RX_RADICES(X_)
+#undef X_
+            }
+          } else {
+            switch (rad) {
+#define X_(r) \
+  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0); break;
+              RX_RADICES(X_)
+#undef X_
+            }
+          }
+          swap();
+          NS *= rad;
+        }
+      }
+    } else {
+      for (int s = s0; s < last; ++s) {
+        const int rad = A.radix[s];
+        const V* t = tw + g.twoff[s];
+        switch (rad) {
+#define X_(r) \
+  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0); break;
+          RX_RADICES(X_)
+#undef X_
+          default: rx_mid_prime<R>(in, out, X, rad, NS, t, t + (s > 0 ? (rad - 1) * NS : 0)); break;
+        }
+        swap();
+        NS *= rad;
+      }
     }
-    if constexpr (KIND == P_C2C) {
+    if constexpr (KIND == P_C2C && BS) {
+      rx_store_c2c<R>(in, X, D);
+    } else if constexpr (KIND == P_C2C) {
       if (fused) {
         const V* t = tw + g.twoff[last];
         switch (A.radix[last]) {

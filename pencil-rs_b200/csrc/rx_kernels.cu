@@ -1,5 +1,6 @@
 // Instantiations and launchers of the runtime-radix pass kernel, one object
-// per kind (RX_KIND: 1 C2C, 2 R2C, 3 C2R, 4 real-to-real).
+// per kind (RX_KIND: 1 C2C, 2 R2C, 3 C2R, 4 real-to-real) and form (RX_BS: 1 for
+// Bluestein passes).
 #include "rx_kernel.cuh"
 
 namespace pb {
@@ -9,19 +10,24 @@ using RxFn = void (*)(const RxArgs);
 
 template <typename R>
 static RxFn<RX_KIND> rx_pick(const PassArgs& A) {
+#if RX_BS
+  (void)A;
+  return rx_kernel<R, RX_KIND, false, true>;
+#else
   if constexpr (RX_KIND == P_C2C)
-    return A.dst_k_contig == 0 ? rx_kernel<R, RX_KIND, true> : rx_kernel<R, RX_KIND, false>;
+    return A.dst_k_contig == 0 ? rx_kernel<R, RX_KIND, true, false> : rx_kernel<R, RX_KIND, false, false>;
   else
-    return rx_kernel<R, RX_KIND, false>;
+    return rx_kernel<R, RX_KIND, false, false>;
+#endif
 }
 
-template <int KIND>
+template <int KIND, bool BS>
 cudaError_t rx_launch_kind(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream);
-template <int KIND>
+template <int KIND, bool BS>
 int rx_occupancy_kind(const RxArgs& X, int real_bytes);
 
 template <>
-cudaError_t rx_launch_kind<RX_KIND>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream) {
+cudaError_t rx_launch_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream) {
   const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem);
   if (err != cudaSuccess) return err;
@@ -30,7 +36,7 @@ cudaError_t rx_launch_kind<RX_KIND>(const RxArgs& X, int real_bytes, int grid, c
 }
 
 template <>
-int rx_occupancy_kind<RX_KIND>(const RxArgs& X, int real_bytes) {
+int rx_occupancy_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes) {
   const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
   int blocks = 0;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem) != cudaSuccess ||

@@ -81,6 +81,7 @@ static int lines_x2(const PassArgs& A) {
 
 bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   std::memset(g, 0, sizeof(*g));
+  g->len = A.bs_m2 ? A.bs_m2 : A.m;
   const int W = real_bytes == 4 ? 2 : 1;
   const int nseq = A.lines * 2 / lines_x2(A);
   int G = std::max(1, (nseq + W - 1) / W);
@@ -90,8 +91,8 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   // contiguous in the destination) hit distinct banks; a transposed store
   // reads whole rows and needs none
   g->P = (A.dst_k_contig != 0 && G > 1) ? G + 1 : G;
-  g->bufv = A.m * g->P;
-  g->pre = (A.kind == P_R2R || A.radix[0] > kRxRegRadix) ? 1 : 0;
+  g->bufv = g->len * g->P;
+  g->pre = (A.kind == P_R2R || A.bs_m2 || A.radix[0] > kRxRegRadix) ? 1 : 0;
   long long tw = 0, ns = 1;
   for (int s = 0; s < A.nstages; ++s) {
     g->twoff[s] = (int)tw;
@@ -138,13 +139,14 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   };
   const bool ok = fits(true, false) || fits(false, false) || fits(true, true) || fits(false, true);
   if (!ok) return false;
-  const long long elems = (long long)nseq * A.m;
+  const long long elems = (long long)nseq * g->len;
   g->threads = elems > 6 * 1024 / (3 - W) ? 512 : elems > 2600 / (3 - W) ? 256 : 128;
   return true;
 }
 
 bool rx_choose(PassArgs& A, int real_bytes, int max_smem, long long max_chunk, long long total_lines, int sms) {
-  const std::vector<int> rad = rx_radices(A.m, real_bytes);
+  const int len = A.bs_m2 ? A.bs_m2 : A.m;
+  const std::vector<int> rad = rx_radices(len, real_bytes);
   if (rad.empty()) return false;
   A.nstages = (int)rad.size();
   for (int s = 0; s < A.nstages; ++s) A.radix[s] = rad[s];
@@ -158,7 +160,7 @@ bool rx_choose(PassArgs& A, int real_bytes, int max_smem, long long max_chunk, l
   // so that a transposed store writes whole 32-byte sectors
   int nseq = min_seq;
   const long long target = real_bytes == 4 ? 2304 : 1152;
-  while (nseq < 128 && (long long)(2 * nseq) * A.m <= target) nseq *= 2;
+  while (nseq < 128 && (long long)(2 * nseq) * len <= target) nseq *= 2;
   if (real_bytes == 4 && nseq < 4) nseq = 4;
   if (real_bytes == 8 && nseq < 2) nseq = 2;
   // no wider than the runs of lines, and enough tiles to fill the device
@@ -177,19 +179,23 @@ bool rx_choose(PassArgs& A, int real_bytes, int max_smem, long long max_chunk, l
 
 namespace pb {
 
-template <int KIND>
+template <int KIND, bool BS>
 cudaError_t rx_launch_kind(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream);
-template <int KIND>
+template <int KIND, bool BS>
 int rx_occupancy_kind(const RxArgs& X, int real_bytes);
-#define RX_DECL(K)                                                                             \
-  template <>                                                                                  \
-  cudaError_t rx_launch_kind<K>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream); \
-  template <>                                                                                  \
-  int rx_occupancy_kind<K>(const RxArgs& X, int real_bytes);
-RX_DECL(1)
-RX_DECL(2)
-RX_DECL(3)
-RX_DECL(4)
+#define RX_DECL(K, B)                                                                                \
+  template <>                                                                                        \
+  cudaError_t rx_launch_kind<K, B>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream);  \
+  template <>                                                                                        \
+  int rx_occupancy_kind<K, B>(const RxArgs& X, int real_bytes);
+RX_DECL(1, false)
+RX_DECL(2, false)
+RX_DECL(3, false)
+RX_DECL(4, false)
+RX_DECL(1, true)
+RX_DECL(2, true)
+RX_DECL(3, true)
+RX_DECL(4, true)
 #undef RX_DECL
 
 static int smem_limit() {
@@ -208,10 +214,18 @@ cudaError_t launch_rx(const PassArgs& A, int real_bytes, cudaStream_t stream) {
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
   switch (A.kind) {
-    case P_C2C: return rx_launch_kind<P_C2C>(X, real_bytes, (int)grid, stream);
-    case P_R2C: return rx_launch_kind<P_R2C>(X, real_bytes, (int)grid, stream);
-    case P_C2R: return rx_launch_kind<P_C2R>(X, real_bytes, (int)grid, stream);
-    case P_R2R: return rx_launch_kind<P_R2R>(X, real_bytes, (int)grid, stream);
+    case P_C2C:
+      return A.bs_m2 ? rx_launch_kind<P_C2C, true>(X, real_bytes, (int)grid, stream)
+                     : rx_launch_kind<P_C2C, false>(X, real_bytes, (int)grid, stream);
+    case P_R2C:
+      return A.bs_m2 ? rx_launch_kind<P_R2C, true>(X, real_bytes, (int)grid, stream)
+                     : rx_launch_kind<P_R2C, false>(X, real_bytes, (int)grid, stream);
+    case P_C2R:
+      return A.bs_m2 ? rx_launch_kind<P_C2R, true>(X, real_bytes, (int)grid, stream)
+                     : rx_launch_kind<P_C2R, false>(X, real_bytes, (int)grid, stream);
+    case P_R2R:
+      return A.bs_m2 ? rx_launch_kind<P_R2R, true>(X, real_bytes, (int)grid, stream)
+                     : rx_launch_kind<P_R2R, false>(X, real_bytes, (int)grid, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -221,10 +235,10 @@ int rx_occupancy(const PassArgs& A, int real_bytes) {
   X.p = A;
   if (!rx_geometry(A, real_bytes, smem_limit(), &X.g)) return 1;
   switch (A.kind) {
-    case P_C2C: return rx_occupancy_kind<P_C2C>(X, real_bytes);
-    case P_R2C: return rx_occupancy_kind<P_R2C>(X, real_bytes);
-    case P_C2R: return rx_occupancy_kind<P_C2R>(X, real_bytes);
-    default: return rx_occupancy_kind<P_R2R>(X, real_bytes);
+    case P_C2C: return A.bs_m2 ? rx_occupancy_kind<P_C2C, true>(X, real_bytes) : rx_occupancy_kind<P_C2C, false>(X, real_bytes);
+    case P_R2C: return A.bs_m2 ? rx_occupancy_kind<P_R2C, true>(X, real_bytes) : rx_occupancy_kind<P_R2C, false>(X, real_bytes);
+    case P_C2R: return A.bs_m2 ? rx_occupancy_kind<P_C2R, true>(X, real_bytes) : rx_occupancy_kind<P_C2R, false>(X, real_bytes);
+    default: return A.bs_m2 ? rx_occupancy_kind<P_R2R, true>(X, real_bytes) : rx_occupancy_kind<P_R2R, false>(X, real_bytes);
   }
 }
 

@@ -22,6 +22,7 @@ constexpr int kRxRegRadix = 16;
 // G vectors of W sequences), the twiddle table, the staged input lines of the
 // tile, tile descriptors and piece rows.
 struct RxGeom {
+  int len;       // FFT length of the stages: m, or the convolution length of a Bluestein pass
   int lgG;       // log2 of the vectors per row
   int P;         // row pitch in vectors
   int threads;

@@ -22,8 +22,8 @@ LIB = os.path.join(PKG, "libpencil_b200.so")
 
 # (source, object, preprocessor definitions): mr_kernels.cu is compiled once
 # per group of lengths (MR_GROUPS in mr_lengths.hpp) and mr_bs_kernels.cu once
-# per kernel kind and layout variant, rx_kernels.cu once per kind, so the
-# groups build in parallel
+# per kernel kind and layout variant, rx_kernels.cu once per kind and
+# form, so the groups build in parallel
 MR_GROUPS = 8
 # the longest compilations first, so that a full build keeps every core busy
 # to the end
@@ -32,7 +32,8 @@ SOURCES = ([("pass_kernel.cu", "pass_kernel.cu.o", [])]
            + [("mr_r2r_kernels.cu", f"mr_r2r_kernels_g{g}.o", [f"-DMR_GROUP={g}"]) for g in range(MR_GROUPS)]
            + [("mr_bs_kernels.cu", f"mr_bs_kernels_k{k}v{v}.o", [f"-DBS_KIND={k}", f"-DBS_V={v}"])
               for k in (1, 2) for v in (0, 1, 2)]
-           + [("rx_kernels.cu", f"rx_kernels_k{k}.o", [f"-DRX_KIND={k}"]) for k in (1, 2, 3, 4)]
+           + [("rx_kernels.cu", f"rx_kernels_k{k}b{b}.o", [f"-DRX_KIND={k}", f"-DRX_BS={b}"])
+              for k in (1, 2, 3, 4) for b in (0, 1)]
            + [(s, s + ".o", []) for s in ("pow2_kernel.cu", "plan.cpp", "field_ops.cu", "aux_kernels.cu",
                                          "no_alloc.cu", "mr_dispatch.cpp", "rx_plan.cpp")])
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
