@@ -4,7 +4,7 @@
 // form of the others: two transforms of the convolution length without leaving
 // shared memory, the chirp and the kernel multiplied in as their first stages
 // read the rows.  Bluestein passes of the generic kernel ran at 0.06-0.17 TB/s
-// (DST-I 100 and 256, DCT-I 384); here 0.23-0.37, and 0.46-0.8 on DCT-II 257
+// (DST-I 100 and 256, DCT-I 384); here 0.27-0.34, and 0.5-0.8 on DCT-II 257
 // and DCT-IV 94.  C2C, R2C and C2R convolutions up to 1024 points keep the
 // compiled kernel (mr_bs.cuh), which is 1.1-1.7 times faster than this one.
 //
@@ -24,6 +24,9 @@
 //   last stage    C2C: butterfly outputs go to memory from registers; the
 //                 other kinds read the finished rows back (the Hermitian
 //                 split, post-twiddles) and store
+//
+// The real-to-real pre- and post-processing works on vectors too: DCT-II of 384
+// f32 lines 1.00 -> 1.50 TB/s against the same code per value.
 //
 // Inverse transforms read their input in reversed index order, X^-1[k] =
 // DFT(x[-q])[k], so only forward butterflies exist.
@@ -111,7 +114,7 @@ __device__ __forceinline__ void rx_stage_lines(E* S, const RxArgs& X, const Tile
     }
   }
   // the missing partner of an odd last line of a pair is zero
-  if ((A.kind == P_R2C || A.kind == P_C2R) && (ta.lines & 1)) {
+  if (A.kind != P_C2C && !(A.kind == P_R2R && A.in_complex) && (ta.lines & 1)) {
     E z;
     memset(&z, 0, sizeof(E));
     for (int q = tid; q < n; q += nt) S[ta.lines * g.sl + q * g.sq] = z;
@@ -379,9 +382,22 @@ __device__ __forceinline__ void rx_put_c2c(typename Cx<R>::T* out, const RxDst& 
   }
 }
 
-// Last stage of a C2C pass, stored from registers.  Transposed: the lanes take
-// the vectors of a row, which are adjacent in the destination row; else
-// consecutive butterflies, whose outputs are adjacent in the destination line.
+// Work item of a store loop over n rows.  Lanes along the vectors of a row for
+// a transposed store, whose row is adjacent in the destination, and for tiles
+// of up to four vectors: a warp then covers at least eight adjacent elements
+// of each line and reads whole rows.  Lanes along the rows otherwise.
+constexpr int kRxWideRow = 2;  // log2 of the vectors
+__device__ __forceinline__ void rx_item(int it, int lgG, int n, unsigned mn, bool tr, int& g, int& k) {
+  if (tr || lgG <= kRxWideRow) {
+    g = it & ((1 << lgG) - 1);
+    k = it >> lgG;
+  } else {
+    g = (int)fdiv(it, n, mn);
+    k = it - g * n;
+  }
+}
+
+// Last stage of a C2C pass, stored from registers.
 template <typename R, int RAD, bool TR>
 __device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const RxV<R>* tw, const RxDst& D) {
   using Q = typename Vec<R>::Q;
@@ -393,13 +409,7 @@ __device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const
   C* out = reinterpret_cast<C*>(X.p.out);
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
     int g, jb;
-    if (TR) {
-      g = it & ((1 << lgG) - 1);
-      jb = it >> lgG;
-    } else {
-      g = (int)fdiv(it, NB, mNB);
-      jb = it - g * NB;
-    }
+    rx_item(it, lgG, NB, mNB, TR, g, jb);
     const int l = g * Vec<R>::W;
     if (l >= D.lines) continue;
     const RxV<R>* p = in + jb * P + g;
@@ -428,18 +438,6 @@ __device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const
       for (int r = 0; r < RAD; ++r)
         rx_put_c2c<R>(out, D, jb + r * NB, l, RxV<R>{qmul(v[r].x, sc), qmul(v[r].y, sc)});
     }
-  }
-}
-
-// Work item of a store loop over n rows: lanes along the vectors of a row for
-// a transposed store, along the rows otherwise.
-__device__ __forceinline__ void rx_item(int it, int lgG, int n, unsigned mn, bool tr, int& g, int& k) {
-  if (tr) {
-    g = it & ((1 << lgG) - 1);
-    k = it >> lgG;
-  } else {
-    g = (int)fdiv(it, n, mn);
-    k = it - g * n;
   }
 }
 
@@ -500,6 +498,29 @@ __device__ __forceinline__ void rx_store_r2c(const RxV<R>* rows, const RxArgs& X
   }
 }
 
+// Output k of 2W adjacent real lines l ..
+template <typename R>
+__device__ __forceinline__ void rx_put_real(R* out, const RxDst& D, int k, int l, const R* v) {
+  constexpr int NV = 2 * Vec<R>::W;
+  if (D.mode == 0) {
+    R* o = out + D.at(k, l);
+    if (l + NV <= D.lines && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+      if constexpr (sizeof(R) == 4)
+        *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+      else
+        *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if (l + j < D.lines) o[j] = v[j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if (l + j < D.lines) out[D.at(k, l + j)] = v[j];
+  }
+}
+
 // C2R: the real and imaginary parts are the two real lines.
 template <typename R>
 __device__ __forceinline__ void rx_store_c2r(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
@@ -524,198 +545,226 @@ __device__ __forceinline__ void rx_store_c2r(const RxV<R>* rows, const RxArgs& X
       v[0] = z.x * sc;
       v[1] = z.y * sc;
     }
-    constexpr int NV = 2 * Vec<R>::W;
-    if (D.mode == 0) {
-      R* o = out + D.at(k, l);
-      if (l + NV <= D.lines && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-        if constexpr (sizeof(R) == 4)
-          *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-        else
-          *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < NV; ++j)
-          if (l + j < D.lines) o[j] = v[j];
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < NV; ++j)
-        if (l + j < D.lines) out[D.at(k, l + j)] = v[j];
-    }
+    rx_put_real<R>(out, D, k, l, v);
   }
 }
 
-// ---- real-to-real kinds: scalar access to the rows (sequence s, element q)
+// ---- real-to-real kinds, a vector of sequences at a time.  A sequence is a
+// pair p: two real lines 2p, 2p + 1 or the parts of complex line p; kinds IV
+// take one sequence per line or part.
+
+__device__ __forceinline__ Q2 rx_q(float a, float b) { return Q2{make_float2(a, b)}; }
+__device__ __forceinline__ float rx_lane(Q2 q, int w) { return w ? q.v.y : q.v.x; }
+__device__ __forceinline__ double rx_lane(double q, int) { return q; }
+template <typename Q>
+__device__ __forceinline__ Q rx_neg(Q a) {
+  return qmul(a, qc<Q>(-1.0));
+}
+
+// Part c of the pairs of vector g at element q of the staged lines.
 template <typename R>
-__device__ __forceinline__ R* rx_slot(RxV<R>* rows, int P, int s, int q) {
-  if constexpr (sizeof(R) == 4)
-    return reinterpret_cast<R*>(rows + q * P + (s >> 1)) + (s & 1);
-  else
-    return reinterpret_cast<R*>(rows + q * P + s);
+__device__ __forceinline__ typename Vec<R>::Q rx_part(const unsigned char* S, const RxArgs& X, int g, int c, int q) {
+  using Q = typename Vec<R>::Q;
+  const PassArgs& A = X.p;
+  const int sl = X.g.sl, o = q * X.g.sq;
+  const R* p = reinterpret_cast<const R*>(S);
+  Q v;
+  if constexpr (sizeof(R) == 4) {
+    if (A.in_complex)
+      v = rx_q(p[2 * (2 * g * sl + o) + c], p[2 * ((2 * g + 1) * sl + o) + c]);
+    else
+      v = rx_q(p[(4 * g + c) * sl + o], p[(4 * g + 2 + c) * sl + o]);
+  } else {
+    v = A.in_complex ? p[2 * (g * sl + o) + c] : p[(2 * g + c) * sl + o];
+  }
+  if (A.pre_mode != W_NONE && weight_hit(A.pre_mode, q, A.n)) v = qmul(v, qc<Q>(A.pre_factor));
+  return v;
+}
+// Element q of the lines (or parts) that are the sequences of vector g, kinds IV.
+template <typename R>
+__device__ __forceinline__ typename Vec<R>::Q rx_line(const unsigned char* S, const RxArgs& X, int g, int q) {
+  using Q = typename Vec<R>::Q;
+  const PassArgs& A = X.p;
+  const int sl = X.g.sl, o = q * X.g.sq;
+  const R* p = reinterpret_cast<const R*>(S);
+  Q v;
+  if constexpr (sizeof(R) == 4) {
+    if (A.in_complex)
+      v = rx_q(p[2 * (g * sl + o)], p[2 * (g * sl + o) + 1]);
+    else
+      v = rx_q(p[2 * g * sl + o], p[(2 * g + 1) * sl + o]);
+  } else {
+    v = A.in_complex ? p[2 * ((g >> 1) * sl + o) + (g & 1)] : p[g * sl + o];
+  }
+  if (A.pre_mode != W_NONE && weight_hit(A.pre_mode, q, A.n)) v = qmul(v, qc<Q>(A.pre_factor));
+  return v;
 }
 template <typename R>
-__device__ __forceinline__ typename Cx<R>::T rx_get(const RxV<R>* rows, int P, int s, int q) {
-  const R* p = rx_slot<R>(const_cast<RxV<R>*>(rows), P, s, q);
-  return mk<typename Cx<R>::T, R>(p[0], p[Vec<R>::W]);
+__device__ __forceinline__ RxV<R> rx_dup(typename Cx<R>::T w) {
+  if constexpr (sizeof(R) == 4)
+    return rx_pack(w.x, w.y, w.x, w.y);
+  else
+    return RxV<R>{w.x, w.y};
 }
 
 // FFT input rows of a real-to-real pass from the staged lines (the
 // definitions of the generic kernel): Makhoul's reordering and pre-twiddle for
 // kinds II / III, the half-length (odd n: zero-padded) form of kinds IV, the
-// symmetric extensions of kinds I.  Sequence s is pair s (two real lines, or
-// the parts of a complex line); kinds IV take one sequence per line or part.
+// symmetric extensions of kinds I.
 template <typename R, int SUB, bool BS>
-__device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows, const RxArgs& X, int lines) {
+__device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows, const RxArgs& X) {
+  using Q = typename Vec<R>::Q;
   using C = typename Cx<R>::T;
   const PassArgs& A = X.p;
-  const int n = A.n, m = A.m, P = X.g.P;
-  const int lgs = X.g.lgG + (sizeof(R) == 4 ? 1 : 0), total = m << lgs;
-  const R pre_f = R(A.pre_factor);
+  const int n = A.n, m = A.m, P = X.g.P, lgG = X.g.lgG, total = m << lgG;
   const C* aux0 = reinterpret_cast<const C*>(A.aux0);
-  const bool cplx = A.in_complex != 0;
-  const R zero = R(0);
-  auto getv = [&](int p, int c, int q) -> R {
-    R v;
-    if (cplx) {
-      v = p < lines ? reinterpret_cast<const R*>(S)[2 * (p * X.g.sl + q * X.g.sq) + c] : zero;
-    } else {
-      const int l = 2 * p + c;
-      v = l < lines ? reinterpret_cast<const R*>(S)[l * X.g.sl + q * X.g.sq] : zero;
-    }
-    if (A.pre_mode != W_NONE && weight_hit(A.pre_mode, q, n)) v *= pre_f;
-    return v;
-  };
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
-    const int s = it & ((1 << lgs) - 1), q = it >> lgs;
-    C z;
+    const int g = it & ((1 << lgG) - 1), q = it >> lgG;
+    RxV<R> z;
     if constexpr (SUB == S_DCT2 || SUB == S_DST2) {
       const int idx = (2 * q < n) ? 2 * q : 2 * (n - 1 - q) + 1;
-      R x = getv(s, 0, idx), y = getv(s, 1, idx);
-      if (SUB == S_DST2 && (idx & 1)) {
-        x = -x;
-        y = -y;
-      }
-      z = mk<C, R>(x, y);
+      z = {rx_part<R>(S, X, g, 0, idx), rx_part<R>(S, X, g, 1, idx)};
+      if (SUB == S_DST2 && (idx & 1)) z = {rx_neg(z.x), rx_neg(z.y)};
     } else if constexpr (SUB == S_DCT3 || SUB == S_DST3) {
       const int i0 = SUB == S_DST3 ? n - 1 - q : q;
-      const R ux = getv(s, 0, i0), uy = getv(s, 1, i0);
-      R vx = zero, vy = zero;
+      const Q ux = rx_part<R>(S, X, g, 0, i0), uy = rx_part<R>(S, X, g, 1, i0);
+      Q vx = qc<Q>(0.0), vy = vx;
       if (q > 0) {
         const int i1 = SUB == S_DST3 ? q - 1 : n - q;
-        vx = getv(s, 0, i1);
-        vy = getv(s, 1, i1);
+        vx = rx_part<R>(S, X, g, 0, i1);
+        vy = rx_part<R>(S, X, g, 1, i1);
       }
-      const C w = aux0[q];
-      const C Vx = cmul(w, mk<C, R>(ux, -vx));
-      const C Vy = cmul(w, mk<C, R>(uy, -vy));
-      z = mk<C, R>(Vx.x - Vy.y, Vx.y + Vy.x);
+      const RxV<R> w = rx_dup<R>(aux0[q]);
+      const RxV<R> Vx = vtw(RxV<R>{ux, rx_neg(vx)}, w), Vy = vtw(RxV<R>{uy, rx_neg(vy)}, w);
+      z = vsubr(Vx, Vy);  // Vx + i Vy
     } else if constexpr (SUB == S_DCT4 || SUB == S_DST4) {
-      const int p = s >> 1, c = s & 1;
       if ((n & 1) == 0) {
         const int i0 = 2 * q, i1 = n - 1 - 2 * q;
         const int j0 = SUB == S_DST4 ? n - 1 - i0 : i0, j1 = SUB == S_DST4 ? n - 1 - i1 : i1;
-        z = cmul(mk<C, R>(getv(p, c, j0), getv(p, c, j1)), aux0[q]);
+        z = vtw(RxV<R>{rx_line<R>(S, X, g, j0), rx_line<R>(S, X, g, j1)}, rx_dup<R>(aux0[q]));
       } else if (q < n) {
-        z = scl(aux0[q], getv(p, c, SUB == S_DST4 ? n - 1 - q : q));
+        const Q x = rx_line<R>(S, X, g, SUB == S_DST4 ? n - 1 - q : q);
+        const RxV<R> w = rx_dup<R>(aux0[q]);
+        z = {qmul(x, w.x), qmul(x, w.y)};
       } else {
-        z = mk<C, R>(zero, zero);
+        z = {qc<Q>(0.0), qc<Q>(0.0)};
       }
     } else if constexpr (SUB == S_DCT1) {
       const int idx = q <= n - 1 ? q : m - q;
-      z = mk<C, R>(getv(s, 0, idx), getv(s, 1, idx));
+      z = {rx_part<R>(S, X, g, 0, idx), rx_part<R>(S, X, g, 1, idx)};
     } else if constexpr (SUB == S_DST1) {
-      if (q == 0 || q == n + 1)
-        z = mk<C, R>(zero, zero);
-      else if (q <= n)
-        z = mk<C, R>(getv(s, 0, q - 1), getv(s, 1, q - 1));
-      else
-        z = mk<C, R>(-getv(s, 0, m - q - 1), -getv(s, 1, m - q - 1));
+      if (q == 0 || q == n + 1) {
+        z = {qc<Q>(0.0), qc<Q>(0.0)};
+      } else {
+        const int idx = q <= n ? q - 1 : m - q - 1;
+        z = {rx_part<R>(S, X, g, 0, idx), rx_part<R>(S, X, g, 1, idx)};
+        if (q > n) z = {rx_neg(z.x), rx_neg(z.y)};
+      }
     } else {  // DHT
-      z = mk<C, R>(getv(s, 0, q), getv(s, 1, q));
+      z = {rx_part<R>(S, X, g, 0, q), rx_part<R>(S, X, g, 1, q)};
     }
-    R* o = rx_slot<R>(rows, P, s, (!BS && A.inv && q != 0) ? m - q : q);
-    o[0] = z.x;
-    o[Vec<R>::W] = z.y;
+    rows[((!BS && A.inv && q != 0) ? m - q : q) * P + g] = z;
   }
 }
 
 // Outputs of a real-to-real pass from the finished rows.
 template <typename R, int SUB>
 __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X, const RxDst& D) {
+  using Q = typename Vec<R>::Q;
   using C = typename Cx<R>::T;
   const PassArgs& A = X.p;
-  const int n = A.n, P = X.g.P;
   constexpr bool iv4 = SUB == S_DCT4 || SUB == S_DST4;
-  const int lgp = X.g.lgG + (sizeof(R) == 4 ? 1 : 0) - (iv4 ? 1 : 0);  // pairs per tile
-  const int total = n << lgp;
+  constexpr int W = Vec<R>::W;
+  const int n = A.n, P = X.g.P, lgG = X.g.lgG, total = n << lgG;
   const unsigned mn = fdiv_magic(n);
-  const R post_f = R(A.post_factor), sc = R(A.scale), h = R(0.5);
+  const Q h = qc<Q>(0.5);
   const C* aux0 = reinterpret_cast<const C*>(A.aux0);
   const C* aux1 = reinterpret_cast<const C*>(A.aux1);
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
-    int p, k;
-    rx_item(it, lgp, n, mn, D.mode == 0, p, k);
-    const int l = A.out_complex ? p : 2 * p;
+    int g, k;
+    rx_item(it, lgG, n, mn, D.mode == 0, g, k);
+    // first destination line of the vector: its values are parts 0 and 1 of W
+    // pairs, or (kinds IV) of W lines or parts
+    const int l = iv4 ? (A.out_complex ? (g * W) >> 1 : g * W) : (A.out_complex ? g * W : 2 * g * W);
     if (l >= D.lines) continue;
-    R v0, v1;
+    double fs = A.scale;
+    if (A.post_mode != W_NONE && weight_hit(A.post_mode, k, n)) fs *= A.post_factor;
+    const Q f = qc<Q>(fs);
+    Q v0, v1 = qc<Q>(0.0);
     if constexpr (SUB == S_DCT2 || SUB == S_DST2 || SUB == S_DHT) {
       const int kk = SUB == S_DST2 ? n - 1 - k : k;
-      const C a = rx_get<R>(rows, P, p, kk), b = rx_get<R>(rows, P, p, kk == 0 ? 0 : n - kk);
-      const C V = mk<C, R>((a.x + b.x) * h, (a.y - b.y) * h), U = mk<C, R>((a.y + b.y) * h, (b.x - a.x) * h);
+      const RxV<R> a = rows[kk * P + g], b = rows[(kk == 0 ? 0 : n - kk) * P + g];
+      // twice the spectra of the pair's two parts
+      const Q vx = qadd(a.x, b.x), vy = qsub(a.y, b.y), ux = qadd(a.y, b.y), uy = qsub(b.x, a.x);
       if constexpr (SUB == S_DHT) {
-        v0 = V.x - V.y;
-        v1 = U.x - U.y;
+        v0 = qmul(qsub(vx, vy), h);
+        v1 = qmul(qsub(ux, uy), h);
       } else {
-        const C w = aux0[kk];
-        v0 = R(2) * (w.x * V.x - w.y * V.y);
-        v1 = R(2) * (w.x * U.x - w.y * U.y);
+        const RxV<R> w = rx_dup<R>(aux0[kk]);
+        v0 = qfma(rx_neg(w.y), vy, qmul(w.x, vx));
+        v1 = qfma(rx_neg(w.y), uy, qmul(w.x, ux));
       }
     } else if constexpr (SUB == S_DCT3 || SUB == S_DST3) {
-      const C z = rx_get<R>(rows, P, p, (k & 1) ? n - 1 - (k >> 1) : (k >> 1));
+      const RxV<R> z = rows[((k & 1) ? n - 1 - (k >> 1) : (k >> 1)) * P + g];
       const bool neg = SUB == S_DST3 && (k & 1);
-      v0 = neg ? -z.x : z.x;
-      v1 = neg ? -z.y : z.y;
+      v0 = neg ? rx_neg(z.x) : z.x;
+      v1 = neg ? rx_neg(z.y) : z.y;
     } else if constexpr (iv4) {
-      auto one = [&](int s) -> R {
-        R v;
-        if ((n & 1) == 0) {
-          if ((k & 1) == 0)
-            v = R(2) * cmul(rx_get<R>(rows, P, s, k >> 1), aux1[k >> 1]).x;
-          else
-            v = R(-2) * cmul(rx_get<R>(rows, P, s, (n - 1 - k) >> 1), aux1[(n - 1 - k) >> 1]).y;
-        } else {
-          v = R(2) * cmul(rx_get<R>(rows, P, s, k), aux1[k]).x;
-        }
-        return (SUB == S_DST4 && (k & 1)) ? -v : v;
-      };
-      v0 = one(2 * p);
-      v1 = one(2 * p + 1);
+      if ((n & 1) == 0) {
+        const int kk = (k & 1) ? (n - 1 - k) >> 1 : k >> 1;
+        const RxV<R> z = vtw(rows[kk * P + g], rx_dup<R>(aux1[kk]));
+        v0 = (k & 1) ? qmul(z.y, qc<Q>(-2.0)) : qmul(z.x, qc<Q>(2.0));
+      } else {
+        v0 = qmul(vtw(rows[k * P + g], rx_dup<R>(aux1[k])).x, qc<Q>(2.0));
+      }
+      if (SUB == S_DST4 && (k & 1)) v0 = rx_neg(v0);
     } else if constexpr (SUB == S_DCT1) {
-      const C z = rx_get<R>(rows, P, p, k);
+      const RxV<R> z = rows[k * P + g];
       v0 = z.x;
       v1 = z.y;
     } else {  // DST-I
-      const C z = rx_get<R>(rows, P, p, k + 1);
-      v0 = -z.y;
+      const RxV<R> z = rows[(k + 1) * P + g];
+      v0 = rx_neg(z.y);
       v1 = z.x;
     }
-    R f = sc;
-    if (A.post_mode != W_NONE && weight_hit(A.post_mode, k, n)) f *= post_f;
-    v0 *= f;
-    v1 *= f;
-    if (A.out_complex) {
-      reinterpret_cast<C*>(A.out)[D.at(k, l)] = mk<C, R>(v0, v1);
-    } else {
-      R* out = reinterpret_cast<R*>(A.out);
-      const long long o = D.at(k, l);
-      if (l + 1 >= D.lines) {
-        out[o] = v0;
-      } else if (D.mode == 0 && (reinterpret_cast<uintptr_t>(out + o) & (2 * sizeof(R) - 1)) == 0) {
-        *reinterpret_cast<C*>(out + o) = mk<C, R>(v0, v1);
+    v0 = qmul(v0, f);
+    v1 = qmul(v1, f);
+    R* out = reinterpret_cast<R*>(A.out);
+    if constexpr (iv4) {
+      // values of sequences gW ..: lines, or parts of a complex line
+      if (A.out_complex) {
+        R* o = out + 2 * D.at(k, l);
+        if constexpr (W == 2)
+          *reinterpret_cast<C*>(o) = mk<C, R>(rx_lane(v0, 0), rx_lane(v0, 1));
+        else
+          o[g & 1] = rx_lane(v0, 0);
       } else {
-        out[o] = v0;
-        out[D.at(k, l + 1)] = v1;
+#pragma unroll
+        for (int w = 0; w < W; ++w)
+          if (l + w < D.lines) out[D.at(k, l + w)] = rx_lane(v0, w);
       }
+    } else if (A.out_complex) {
+      C* oc = reinterpret_cast<C*>(A.out);
+      if constexpr (W == 2) {
+        const C a = mk<C, R>(rx_lane(v0, 0), rx_lane(v1, 0)), b = mk<C, R>(rx_lane(v0, 1), rx_lane(v1, 1));
+        const long long o = D.at(k, l);
+        if (D.mode == 0) {
+          rx_put2(reinterpret_cast<float2*>(oc + o), a, b, l + 1 < D.lines);
+        } else {
+          oc[o] = a;
+          if (l + 1 < D.lines) oc[D.at(k, l + 1)] = b;
+        }
+      } else {
+        oc[D.at(k, l)] = mk<C, R>(rx_lane(v0, 0), rx_lane(v1, 0));
+      }
+    } else {
+      R v[2 * W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        v[2 * w] = rx_lane(v0, w);
+        v[2 * w + 1] = rx_lane(v1, w);
+      }
+      rx_put_real<R>(out, D, k, l, v);
     }
   }
 }
@@ -790,7 +839,7 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
       s0 = 0;
       switch (A.sub) {
 #define X_(u) \
-  case u: rx_pre_r2r<R, u, BS>(S, b0, X, ta.lines); break;
+  case u: rx_pre_r2r<R, u, BS>(S, b0, X); break;
         RX_SUBS(X_)
 #undef X_
       }

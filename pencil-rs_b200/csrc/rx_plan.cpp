@@ -87,10 +87,10 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   int G = std::max(1, (nseq + W - 1) / W);
   while ((1 << g->lgG) < G) ++g->lgG;
   G = 1 << g->lgG;
-  // an odd row pitch lets lanes that walk along the rows (the stores of lines
-  // contiguous in the destination) hit distinct banks; a transposed store
-  // reads whole rows and needs none
-  g->P = (A.dst_k_contig != 0 && G > 1) ? G + 1 : G;
+  // an odd row pitch lets lanes that walk along the rows (stores to lines
+  // contiguous in the destination from tiles of more than four vectors) hit
+  // distinct banks; the other stores read whole rows and need none
+  g->P = (A.dst_k_contig != 0 && G > 4) ? G + 1 : G;
   g->bufv = g->len * g->P;
   g->pre = (A.kind == P_R2R || A.bs_m2 || A.radix[0] > kRxRegRadix) ? 1 : 0;
   long long tw = 0, ns = 1;
