@@ -253,20 +253,18 @@ __host__ __device__ constexpr int mr_bs_min_ctas(int real_bytes, int N) {
 template <typename R, int N, int K, int V>
 __global__ void __launch_bounds__(MR_THREADS, mr_bs_min_ctas((int)sizeof(R), N)) mr_bs_kernel(const PassArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   mr_run<R, N, false, V == 1, V != 0, 0, K>(A, blockIdx.x, gridDim.x, A.ntiles, smem, true);
 }
 
 template <typename R, int N, int K, int V>
 cudaError_t mr_bs_launch(const PassArgs& A, cudaStream_t stream) {
   constexpr size_t smem = mr_smem_bytes<R, N>();
-  cudaError_t err =
-      cudaFuncSetAttribute(mr_bs_kernel<R, N, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = pb_allow_smem<mr_bs_kernel<R, N, K, V>>((int)smem);
   if (err != cudaSuccess) return err;
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
-  mr_bs_kernel<R, N, K, V><<<dim3((unsigned)grid), MR_THREADS, smem, stream>>>(A);
-  return cudaGetLastError();
+  return pb_launch<PassArgs>(mr_bs_kernel<R, N, K, V>, grid, MR_THREADS, smem, stream, A);
 }
 
 template <typename R, int N, int K, int V>

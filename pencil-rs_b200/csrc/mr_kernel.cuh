@@ -32,6 +32,7 @@
 #include "pb_aux.hpp"
 #include "pb_device.cuh"
 #include "pb_fft.cuh"
+#include "pb_launch.cuh"
 #include "smem_layout.hpp"
 
 namespace pb {
@@ -703,6 +704,11 @@ __device__ __forceinline__ void mr_run(const PassArgs& A, long long first, long 
       for (int k = tid; k < nout; k += MR_THREADS) ktab[k] = A.ktab[k];
   }
   TileAddr ta = load_tile(tiles, tile);
+  TileAddr t1 = ta;
+  if (tile + step < end) t1 = load_tile(tiles, tile + step);
+  PieceAddr my_piece{0, 0};
+  if (tid < npieces) my_piece = pieces[tile * npieces + tid];
+  pb_dependency_wait(ta.src0, t1.src0);  // the tables above belong to the plan; the data is read from here on
   C v[G::U0][G::R0];
   if constexpr (BS != 0)
     mr_load_bs<R, N, BS, SX>(v, A, ta);
@@ -710,14 +716,11 @@ __device__ __forceinline__ void mr_run(const PassArgs& A, long long first, long 
     mr_load_r2r<R, N, SX>(v, A, ta);
   else
     mr_load<R, N, SX, S>(v, A, ta);
-  TileAddr t1 = ta;
-  if (tile + step < end) t1 = load_tile(tiles, tile + step);
-  PieceAddr my_piece{0, 0};
-  if (tid < npieces) my_piece = pieces[tile * npieces + tid];
   __syncthreads();  // twiddles and k table in place
 
   for (;;) {
     const bool has_next = tile + step < end;
+    if (!has_next && setup) pb_allow_successor();
     TileAddr t2 = t1;
     PieceAddr next_piece{0, 0};
     C nv[G::U0][G::R0];
@@ -764,7 +767,7 @@ __device__ __forceinline__ void mr_run(const PassArgs& A, long long first, long 
 template <typename R, int N, int V, int S = 0>
 __global__ void __launch_bounds__(MR_THREADS, mr_min_ctas((int)sizeof(R), N, S)) mr_kernel(const PassArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   mr_run<R, N, false, V == 1, V != 0, S>(A, blockIdx.x, gridDim.x, A.ntiles, smem, true);
 }
 
@@ -786,12 +789,13 @@ cudaError_t mr_launch_s(const PassArgs& A, cudaStream_t stream) {
   constexpr size_t smem = mr_smem_bytes<R, N>();
   const int var = mr_variant(A);
   const auto kern = var == 1 ? mr_kernel<R, N, 1, S> : var == 2 ? mr_kernel<R, N, 2, S> : mr_kernel<R, N, 0, S>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = var == 1   ? pb_allow_smem<mr_kernel<R, N, 1, S>>((int)smem)
+                    : var == 2 ? pb_allow_smem<mr_kernel<R, N, 2, S>>((int)smem)
+                               : pb_allow_smem<mr_kernel<R, N, 0, S>>((int)smem);
   if (err != cudaSuccess) return err;
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
-  kern<<<dim3((unsigned)grid), MR_THREADS, smem, stream>>>(A);
-  return cudaGetLastError();
+  return pb_launch<PassArgs>(kern, grid, MR_THREADS, smem, stream, A);
 }
 
 // Host entry points of one length (instantiated by mr_kernels.cu): the

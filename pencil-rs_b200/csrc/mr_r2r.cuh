@@ -368,7 +368,7 @@ __device__ __forceinline__ void mr_tile_r2r(const PassArgs& A, const TileAddr& t
 template <typename R, int N, int V>
 __global__ void __launch_bounds__(MR_THREADS, mr_r2r_min_ctas((int)sizeof(R), N)) mr_r2r_kernel(const PassArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   mr_run<R, N, true, V == 1>(A, blockIdx.x, gridDim.x, A.ntiles, smem, true);
 }
 
@@ -376,12 +376,12 @@ template <typename R, int N>
 cudaError_t mr_r2r_launch(const PassArgs& A, cudaStream_t stream) {
   constexpr size_t smem = mr_smem_bytes<R, N, true>();
   const auto kern = A.src_k_contig == 0 ? mr_r2r_kernel<R, N, 1> : mr_r2r_kernel<R, N, 0>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = A.src_k_contig == 0 ? pb_allow_smem<mr_r2r_kernel<R, N, 1>>((int)smem)
+                                        : pb_allow_smem<mr_r2r_kernel<R, N, 0>>((int)smem);
   if (err != cudaSuccess) return err;
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
-  kern<<<dim3((unsigned)grid), MR_THREADS, smem, stream>>>(A);
-  return cudaGetLastError();
+  return pb_launch<PassArgs>(kern, grid, MR_THREADS, smem, stream, A);
 }
 
 // resident CTAs per SM, the smaller of the two variants' figures

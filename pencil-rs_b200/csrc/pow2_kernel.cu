@@ -24,6 +24,7 @@
 #include "pb_aux.hpp"
 #include "pb_device.cuh"
 #include "pb_fft.cuh"
+#include "pb_launch.cuh"
 #include "smem_layout.hpp"
 
 namespace pb {
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(P2_THREADS, 2) pow2_kernel(const PassArgs A) {
   PieceAddr* prow = reinterpret_cast<PieceAddr*>(ktab + NOUT);
   long long* Jtab = reinterpret_cast<long long*>(prow + P2_MAX_PIECES);
 
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   const long long G0 = gridDim.x;
   long long tile = blockIdx.x;
   if (tile >= A.ntiles) return;
@@ -443,19 +444,21 @@ __global__ void __launch_bounds__(P2_THREADS, 2) pow2_kernel(const PassArgs A) {
   // tile descriptors are fetched two tiles ahead and piece rows one tile
   // ahead, so the prefetch of a tile never waits on the load of its address
   TileAddr ta = load_tile(tiles, tile);
+  TileAddr t1 = ta;
+  if (tile + G0 < A.ntiles) t1 = load_tile(tiles, tile + G0);
+  PieceAddr my_piece{0, 0};
+  if (tid < npieces) my_piece = pieces[tile * npieces + tid];
+  pb_dependency_wait(ta.src0, t1.src0);
   C v[LPT][8];
   {
     P2Raw<R, KIND, LPT, FH> raw;
     p2_fetch<R, N, KIND, LPT, FH, SX>(raw, A, ta, fs, fc);
     p2_finish<R, N, KIND, LPT, FH>(v, raw, A, fc);
   }
-  TileAddr t1 = ta;
-  if (tile + G0 < A.ntiles) t1 = load_tile(tiles, tile + G0);
-  PieceAddr my_piece{0, 0};
-  if (tid < npieces) my_piece = pieces[tile * npieces + tid];
 
   for (;;) {
     const bool has_next = tile + G0 < A.ntiles;
+    if (!has_next) pb_allow_successor();
     TileAddr t2 = t1;
     PieceAddr next_piece{0, 0};
     P2Raw<R, KIND, LPT, FH> nraw;
@@ -768,7 +771,7 @@ __global__ void __launch_bounds__(P2_THREADS, 2) pow2_half_c2r_kernel(const Pass
   extern __shared__ __align__(16) unsigned char smem[];
   C* sm = reinterpret_cast<C*>(smem);
 
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   const long long G0 = gridDim.x;
   long long tile = blockIdx.x;
   if (tile >= A.ntiles) return;
@@ -858,17 +861,19 @@ __global__ void __launch_bounds__(P2_THREADS, 2) pow2_half_c2r_kernel(const Pass
   };
 
   TileAddr ta = load_tile(tiles, tile);
+  TileAddr t1 = ta;
+  if (tile + G0 < A.ntiles) t1 = load_tile(tiles, tile + G0);
+  pb_dependency_wait(ta.src0, t1.src0);
   C v[2][8];
   {
     Raw raw;
     fetch(raw, ta);
     finish(v, raw);
   }
-  TileAddr t1 = ta;
-  if (tile + G0 < A.ntiles) t1 = load_tile(tiles, tile + G0);
 
   for (;;) {
     const bool has_next = tile + G0 < A.ntiles;
+    if (!has_next) pb_allow_successor();
     TileAddr t2 = t1;
     Raw nraw;
     if (has_next) {
@@ -969,12 +974,12 @@ static cudaError_t p2_launch(const PassArgs& A, cudaStream_t stream) {
   // strided source lines (the tile's lines adjacent along the source's innermost axis)
   auto fn = A.src_k_contig == 0 ? pow2_kernel<R, N, KIND, INV, DIRECT, true, DSPLIT>
                                 : pow2_kernel<R, N, KIND, INV, DIRECT, false, DSPLIT>;
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = A.src_k_contig == 0 ? pb_allow_smem<pow2_kernel<R, N, KIND, INV, DIRECT, true, DSPLIT>>((int)smem)
+                                        : pb_allow_smem<pow2_kernel<R, N, KIND, INV, DIRECT, false, DSPLIT>>((int)smem);
   if (err != cudaSuccess) return err;
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
-  fn<<<dim3((unsigned)grid), P2_THREADS, smem, stream>>>(A);
-  return cudaGetLastError();
+  return pb_launch<PassArgs>(fn, grid, P2_THREADS, smem, stream, A);
 }
 
 template <typename R, int N>
@@ -1077,12 +1082,11 @@ template <int M>
 static cudaError_t p2h_launch(const PassArgs& A, cudaStream_t stream) {
   const size_t smem = p2h_smem<M>();
   auto fn = pow2_half_c2r_kernel<M>;
-  cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = pb_allow_smem<pow2_half_c2r_kernel<M>>((int)smem);
   if (err != cudaSuccess) return err;
   long long grid = A.grid_ctas > 0 ? A.grid_ctas : A.ntiles;
   if (grid > A.ntiles) grid = A.ntiles;
-  fn<<<dim3((unsigned)grid), P2_THREADS, smem, stream>>>(A);
-  return cudaGetLastError();
+  return pb_launch<PassArgs>(fn, grid, P2_THREADS, smem, stream, A);
 }
 
 template <int M>

@@ -46,6 +46,7 @@
 #include <cuda_runtime.h>
 
 #include "pb_device.cuh"
+#include "pb_launch.cuh"
 #include "rx_fft.cuh"
 #include "rx_plan.hpp"
 
@@ -781,7 +782,7 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
   using V = RxV<R>;
   const PassArgs& A = X.p;
   const RxGeom& g = X.g;
-  if (A.gate != nullptr && *A.gate != 0) return;
+  if (pb_rejected(A.gate)) return;
   long long tile = blockIdx.x;
   const long long step = gridDim.x, end = A.ntiles;
   if (tile >= end) return;
@@ -813,6 +814,7 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
   if (tid < np) prow[tid] = pieces[tile * np + tid];
   for (int i = tid; i < g.tw_smem; i += nt) W[i] = Wg[i];
   __syncthreads();
+  pb_dependency_wait();  // the tables above belong to the plan; the data is read from here on
   rx_stage<R, KIND>(S, X, desc[0]);
   rx_cp_commit();
 
@@ -859,6 +861,7 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
     }
     __syncthreads();
     const bool has_next = tile + step < end;
+    if (!has_next) pb_allow_successor();
     if (has_next) {
       if (!g.alias) rx_stage<R, KIND>(S, X, tn);
       if (tid == 0 && tile + 2 * step < end) {

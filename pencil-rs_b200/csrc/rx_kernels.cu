@@ -21,6 +21,18 @@ static RxFn<RX_KIND> rx_pick(const PassArgs& A) {
 #endif
 }
 
+// the device's whole shared memory: tiles of any length may be launched
+template <typename R>
+static cudaError_t rx_allow_smem(const RxArgs& X) {
+#if RX_BS
+  return pb_allow_smem<rx_kernel<R, RX_KIND, false, true>>(X.g.max_smem);
+#else
+  if constexpr (RX_KIND == P_C2C)
+    if (X.p.dst_k_contig == 0) return pb_allow_smem<rx_kernel<R, RX_KIND, true, false>>(X.g.max_smem);
+  return pb_allow_smem<rx_kernel<R, RX_KIND, false, false>>(X.g.max_smem);
+#endif
+}
+
 template <int KIND, bool BS>
 cudaError_t rx_launch_kind(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream);
 template <int KIND, bool BS>
@@ -29,17 +41,16 @@ int rx_occupancy_kind(const RxArgs& X, int real_bytes);
 template <>
 cudaError_t rx_launch_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream) {
   const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem);
+  const cudaError_t err = real_bytes == 4 ? rx_allow_smem<float>(X) : rx_allow_smem<double>(X);
   if (err != cudaSuccess) return err;
-  kern<<<dim3((unsigned)grid), X.g.threads, X.g.smem, stream>>>(X);
-  return cudaGetLastError();
+  return pb_launch<RxArgs>(kern, grid, X.g.threads, X.g.smem, stream, X);
 }
 
 template <>
 int rx_occupancy_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes) {
   const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
   int blocks = 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, X.g.smem) != cudaSuccess ||
+  if ((real_bytes == 4 ? rx_allow_smem<float>(X) : rx_allow_smem<double>(X)) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, X.g.threads, X.g.smem) != cudaSuccess)
     return 1;
   return blocks > 0 ? blocks : 1;

@@ -3,6 +3,7 @@
 #include "rx_plan.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -81,6 +82,7 @@ static int lines_x2(const PassArgs& A) {
 
 bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   std::memset(g, 0, sizeof(*g));
+  g->max_smem = max_smem;
   g->len = A.bs_m2 ? A.bs_m2 : A.m;
   const int W = real_bytes == 4 ? 2 : 1;
   const int nseq = A.lines * 2 / lines_x2(A);
@@ -198,12 +200,17 @@ RX_DECL(3, true)
 RX_DECL(4, true)
 #undef RX_DECL
 
+// The current device's shared memory per block, looked up once per device.
 static int smem_limit() {
+  static std::atomic<int> known[64];
   int dev = 0, optin = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess && optin > 0)
-    return optin;
-  return 227 * 1024;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 227 * 1024;
+  optin = known[dev].load(std::memory_order_relaxed);
+  if (optin > 0) return optin;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || optin <= 0)
+    return 227 * 1024;
+  known[dev].store(optin, std::memory_order_relaxed);
+  return optin;
 }
 
 cudaError_t launch_rx(const PassArgs& A, int real_bytes, cudaStream_t stream) {

@@ -33,6 +33,7 @@ struct RxGeom {
   int sl, sq;    // staging strides of a line and of an element, in elements
   int off_tw, off_stage, off_desc;  // byte offsets in shared memory
   int smem;      // bytes
+  int max_smem;  // the device's limit
   int twoff[kRxMaxStages];
 };
 
