@@ -45,12 +45,14 @@ struct R2rSource {
 
 // Line length n of kind SUB on an N-point FFT: N for the DHT and the type-II
 // and type-III kinds, N/2 + 1 for DCT-I, N/2 - 1 for DST-I, 2N for the type-IV
-// kinds.
+// kinds, N + 1 and N - 1 for the odd-N forms of DCT-I and DST-I.
 template <int N, int SUB>
 __host__ __device__ constexpr int r2r_len() {
   return SUB == S_DCT1   ? N / 2 + 1
          : SUB == S_DST1 ? N / 2 - 1
          : (SUB == S_DCT4 || SUB == S_DST4) ? 2 * N
+         : SUB == S_DCT1_ODD                 ? N + 1
+         : SUB == S_DST1_ODD                 ? N - 1
                                              : N;
 }
 
@@ -99,6 +101,59 @@ __device__ __forceinline__ void mr_load_r2r_iv(typename Cx<R>::T (&v)[MRGeom<R, 
         if (weight_hit(A.pre_mode, j1, n)) x1 *= pf;
       }
       v[u][r] = cmul(mk<C, R>(x0, x1), aux0[q]);
+    }
+  }
+}
+
+// Type-I kinds whose N = n - 1 (DCT-I) or n + 1 (DST-I) is odd: one N-point FFT
+// per real line (or component of a complex line) instead of one 2N-point FFT
+// per pair.  The 2N-point DFT of the symmetric extension splits into
+// N-point ones without twiddles (2 and N are coprime): its even outputs are the
+// DFT of c_j = x_j -+ x_{N-j}, its odd ones, taken as k + N, that of
+// b_j = (-1)^j (x_j +- x_{N-j}) (upper signs DST-I, whose x_0 = x_N = 0; the
+// line's elements are x_1 ..).  Both DFTs are purely imaginary (DST-I) or real
+// (DCT-I), so z = c + i b carries both: output k of the line is a part of
+// Z[k/2] (even k) or Z[(k+N)/2] (odd k).
+template <typename R, int N, int SUB, bool SX>
+__device__ __forceinline__ void mr_load_r2r_odd(typename Cx<R>::T (&v)[MRGeom<R, N>::U0][MRGeom<R, N>::R0],
+                                                const PassArgs& A, const TileAddr& ta) {
+  using C = typename Cx<R>::T;
+  using G = MRGeom<R, N>;
+  constexpr int NB = G::NB0;
+  constexpr int R0 = G::R0;
+  constexpr int n = r2r_len<N, SUB>();
+  constexpr bool DST = SUB == S_DST1_ODD;
+  const R zero = R(0);
+  const int L = ta.lines;
+  const bool cplx = A.in_complex != 0;
+  const R* __restrict__ inr = reinterpret_cast<const R*>(A.in);
+  const R pf = R(A.pre_factor);
+#pragma unroll
+  for (int u = 0; u < G::U0; ++u) {
+    const int b = threadIdx.x + u * MR_THREADS;
+    const int s = SX ? b % G::NSEQ : b / NB;
+    const int jb = SX ? b / G::NSEQ : b - s * NB;
+    const int p = s >> 1, c = s & 1;
+    const bool live = (G::B0 % MR_THREADS == 0) || b < G::B0;
+    const bool ok = live && (cplx ? p < L : 2 * p + c < L);
+    const long long base = cplx ? 2 * (ta.src0 + (long long)p * ta.srcb) + c : ta.src0 + (long long)(2 * p + c) * ta.srcb;
+    const long long step = (cplx ? 2 : 1) * (SX ? (long long)ta.srcq : 1LL);
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      const int q = jb + r * NB;
+      // x_q and x_{N-q}: elements q and N - q of a DCT-I line, q - 1 and
+      // N - q - 1 of a DST-I line (x_0 = 0)
+      const int j0 = DST ? q - 1 : q, j1 = DST ? N - q - 1 : N - q;
+      const bool in = ok && (!DST || q > 0);
+      R x0 = in ? inr[base + j0 * step] : zero;
+      R x1 = in ? inr[base + j1 * step] : zero;
+      if (A.pre_mode != W_NONE) {
+        if (weight_hit(A.pre_mode, j0, n)) x0 *= pf;
+        if (weight_hit(A.pre_mode, j1, n)) x1 *= pf;
+      }
+      const R sum = x0 + x1, dif = x0 - x1;
+      const R bq = DST ? sum : dif;
+      v[u][r] = mk<C, R>(DST ? dif : sum, (q & 1) ? -bq : bq);
     }
   }
 }
@@ -195,6 +250,12 @@ __device__ __forceinline__ void mr_load_r2r(typename Cx<R>::T (&v)[MRGeom<R, N>:
     case S_DST1:
       if constexpr (N % 2 == 0) mr_load_r2r_k<R, N, S_DST1, SX>(v, A, ta);
       break;
+    case S_DCT1_ODD:
+      if constexpr (N % 2 == 1) mr_load_r2r_odd<R, N, S_DCT1_ODD, SX>(v, A, ta);
+      break;
+    case S_DST1_ODD:
+      if constexpr (N % 2 == 1) mr_load_r2r_odd<R, N, S_DST1_ODD, SX>(v, A, ta);
+      break;
     case S_DCT4: mr_load_r2r_iv<R, N, S_DCT4, SX>(v, A, ta); break;
     case S_DST4: mr_load_r2r_iv<R, N, S_DST4, SX>(v, A, ta); break;
     default: mr_load_r2r_k<R, N, S_DHT, SX>(v, A, ta); break;
@@ -243,6 +304,18 @@ __device__ __forceinline__ typename Cx<R>::T r2r_output(const typename Cx<R>::T*
       const C z = seq[G::pad((k & 1) ? n - 1 - (k >> 1) : (k >> 1))];
       return (sub == S_DST3 && (k & 1)) ? mk<C, R>(-z.x, -z.y) : z;
     }
+    case S_DCT1_ODD:
+    case S_DST1_ODD: {
+      // DCT-I: Re Z[k/2] (even k), Im Z[(k+N)/2 mod N] (odd k); DST-I with
+      // k + 1 for k: -Im Z, Re Z
+      const int kk = sub == S_DST1_ODD ? k + 1 : k;
+      const bool odd = (kk & 1) != 0;
+      int i = odd ? (kk + N) >> 1 : kk >> 1;
+      if (sub == S_DCT1_ODD && i == N) i = 0;
+      const C u0 = seq[G::pad(i)], u1 = seq[G::SEQ + G::pad(i)];
+      if (sub == S_DST1_ODD) return odd ? mk<C, R>(u0.x, u1.x) : mk<C, R>(-u0.y, -u1.y);
+      return odd ? mk<C, R>(u0.y, u1.y) : mk<C, R>(u0.x, u1.x);
+    }
     case S_DCT1: return seq[G::pad(k)];
     case S_DST1: {
       const C z = seq[G::pad(k + 1)];
@@ -265,8 +338,9 @@ __device__ __forceinline__ void mr_store_r2r_k(const PassArgs& A, const TileAddr
                                                const long long* Atab) {
   using C = typename Cx<R>::T;
   using G = MRGeom<R, N>;
-  // pairs of the tile: one FFT sequence each, two for the type-IV kinds
-  constexpr bool IV = SUB == S_DCT4 || SUB == S_DST4;
+  // pairs of the tile: one FFT sequence each, two for the type-IV kinds and the
+  // odd-N forms of type I
+  constexpr bool IV = r2r_seq_per_line(SUB);
   constexpr int NSEQ = IV ? G::NSEQ / 2 : G::NSEQ;
   constexpr int SEQ = IV ? 2 * G::SEQ : G::SEQ;
   constexpr int n = r2r_len<N, SUB>();
@@ -334,6 +408,12 @@ __device__ __forceinline__ void mr_store_r2r(const PassArgs& A, const TileAddr& 
       break;
     case S_DST1:
       if constexpr (N % 2 == 0) mr_store_r2r_k<R, N, S_DST1>(A, ta, res, Atab);
+      break;
+    case S_DCT1_ODD:
+      if constexpr (N % 2 == 1) mr_store_r2r_k<R, N, S_DCT1_ODD>(A, ta, res, Atab);
+      break;
+    case S_DST1_ODD:
+      if constexpr (N % 2 == 1) mr_store_r2r_k<R, N, S_DST1_ODD>(A, ta, res, Atab);
       break;
     case S_DCT4: mr_store_r2r_k<R, N, S_DCT4>(A, ta, res, Atab); break;
     case S_DST4: mr_store_r2r_k<R, N, S_DST4>(A, ta, res, Atab); break;

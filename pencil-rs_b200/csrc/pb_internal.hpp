@@ -38,7 +38,16 @@ enum R2rSub : int {
   S_DCT1 = 0, S_DCT2 = 1, S_DCT3 = 2, S_DCT4 = 3,
   S_DST1 = 4, S_DST2 = 5, S_DST3 = 6, S_DST4 = 7,
   S_DHT = 8,
+  // the type-I kinds as one N-point FFT per line, N = n + 1 (DST-I) or n - 1
+  // (DCT-I) odd (the register kernels' forms of S_DST1 and S_DCT1)
+  S_DST1_ODD = 9, S_DCT1_ODD = 10,
 };
+
+// Whether a real-to-real form takes an FFT sequence per real line (or
+// component of a complex line) instead of one per pair.
+PB_HD constexpr bool r2r_seq_per_line(int sub) {
+  return sub == S_DCT4 || sub == S_DST4 || sub == S_DST1_ODD || sub == S_DCT1_ODD;
+}
 
 // Weight modes: diagonal factors applied to line inputs (pre) or outputs
 // (post); used by the adjoint (VJP) variants.
@@ -85,7 +94,7 @@ struct PassArgs {
   double scale;
   int src_k_contig;  // transform axis has unit stride in the source
   int dst_k_contig;  // transform axis has unit stride in the destination (register kernel: 2 = and is split across ranks)
-  int fast;          // 1: power-of-two kernel (pow2_kernel.cu), 2: mixed-radix (mr_kernel.cuh), 3: its R2R kinds (mr_r2r.cuh)
+  int fast;          // 1: power-of-two kernel (pow2_kernel.cu), 2: mixed-radix (mr_kernel.cuh), 3: its R2R kinds (mr_r2r.cuh), 4: its Bluestein passes (mr_bs.cuh), 5: runtime radices (rx_kernel.cuh)
   int half;          // fast == 1, C2R: one real line as an m-point complex sequence (m = N/2; aux0 = W_N^c, c <= m/16)
   int nstages;
   int radix[MAXSTAGES];

@@ -1201,6 +1201,21 @@ static void build_fast_tables(pb_plan& P, PassArgs& A, const Pencil& src, const 
   set_grid(P, A);
 }
 
+// Whether the register kernel runs a type-I kind of 2N points (N odd) in its
+// N-point form: where that is the only one it has; in f64 where it saves a
+// stage (2N = 770: 4 stages, N = 385: 3, DST-I 384 1.14 -> 1.35 TB/s; at equal
+// counts it lost 4-19%); in f32 at equal counts where the 2N-point schedule
+// has a radix of 14 or more, which spills (DCT-I 106 0.98 -> 1.38 TB/s, DST-I 62
+// 1.20 -> 1.44, 48 1.16 -> 1.45; with smaller radices it lost up to 31%).
+static bool odd_form_pays(int m, int real_bytes) {
+  if (!mr_r2r_supported(m / 2, real_bytes)) return false;
+  if (!mr_r2r_supported(m, real_bytes)) return true;
+  int full[12], half[12];
+  const int nf = mr_r2r_radices(m, real_bytes, full, 12), nh = mr_r2r_radices(m / 2, real_bytes, half, 12);
+  if (real_bytes == 8) return nh < nf;
+  return nh == nf && *std::max_element(full, full + nf) >= 14;
+}
+
 // One fused pass for `st` under `op` from layout `src` to layout `dst`.
 static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Pencil& src, const Pencil& dst,
                       bool in_complex, bool out_complex) {
@@ -1340,19 +1355,31 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
   }
   // real-to-real kinds on the mixed-radix kernel (the type-IV kinds for even
   // n): contiguous or strided source lines, a direct or transposed store, FFT
-  // lengths of kMrR2rLengths
-  const bool iv4 = op.sub == S_DCT4 || op.sub == S_DST4;
+  // lengths of kMrR2rLengths.  The type-I kinds whose symmetric extension has
+  // 2N points with N odd take their N-point form where N is such a length.
   const bool r2r_strided = src.perm[N - 1] == b && b != a;
+  const int odd_sub = op.kind != P_R2R || A.n % 2 != 0 || A.n < 4 ? -1
+                      : op.sub == S_DST1                          ? S_DST1_ODD
+                      : op.sub == S_DCT1                          ? S_DCT1_ODD
+                                                                  : -1;
+  const bool iv4 = op.sub == S_DCT4 || op.sub == S_DST4;
+  const bool odd1 = odd_sub >= 0 && odd_form_pays(A.m, P.real_bytes);
   if (!A.fast && !P.force_generic && op.kind == P_R2R && (!iv4 || A.n % 2 == 0) &&
-      mr_r2r_supported(A.m, P.real_bytes) && (src.perm[N - 1] == a || r2r_strided) && src.split_of(a) < 0) {
+      (odd1 || mr_r2r_supported(A.m, P.real_bytes)) && (src.perm[N - 1] == a || r2r_strided) && src.split_of(a) < 0) {
     const bool direct = dst.perm[N - 1] == a && dst.split_of(a) < 0;
     const int ta = dst.split_of(a);
     const bool transposed = !direct && dst.perm[N - 1] == b && (ta < 0 || dst.grid[ta] <= 64);
     if (direct || transposed) {
       A.fast = 3;
       A.dst_k_contig = direct ? 1 : 0;
-      // a pair of lines per FFT sequence; the type-IV kinds take a sequence per line
-      L = mr_r2r_lines(A.m, in_complex ? 1 : 0, P.real_bytes) / (iv4 ? 2 : 1);
+      if (odd1) {
+        A.sub = odd_sub;
+        A.m /= 2;
+        A.bs_m2 = 0;
+        A.twiddle = enc(roots_table(P, A.m));
+      }
+      // a pair of lines per FFT sequence, or a sequence per line
+      L = mr_r2r_lines(A.m, in_complex ? 1 : 0, P.real_bytes) / (r2r_seq_per_line(A.sub) ? 2 : 1);
       A.lines = L;
     }
   }
@@ -1384,13 +1411,13 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
     const bool transposed = !direct && dst.perm[N - 1] == b && (ta < 0 || dst.grid[ta] <= kRxMaxPieces);
     const bool dsplit = !direct && dst.perm[N - 1] == a && ta >= 0 && dst.grid[ta] <= kRxMaxPieces;
     if (direct || transposed || dsplit) {
-      PassArgs B = A;
-      B.dst_k_contig = direct ? 1 : (dsplit ? 2 : 0);
       long long run = 0, lines = P.extra;
       for (size_t i = 0; i + 1 < cuts.size(); ++i) run = std::max(run, cuts[i + 1] - cuts[i]);
       for (int x = 0; x < N; ++x)
         if (x != a) lines *= src.shape[x];
-      if (rx_choose(B, P.real_bytes, P.max_smem, run, lines, device_sms())) {
+      auto take = [&](PassArgs B) {
+        B.dst_k_contig = direct ? 1 : (dsplit ? 2 : 0);
+        if (!rx_choose(B, P.real_bytes, P.max_smem, run, lines, device_sms())) return false;
         A = B;
         A.fast = 5;
         A.twiddle = enc(rx_table(P, A));
@@ -1399,7 +1426,17 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
           A.bs_kernel = enc(rx_vectors(P, bluestein_kernel_table(P, A.m, A.bs_m2, A.inv), A.bs_m2));
         }
         L = A.lines;
+        return true;
+      };
+      bool taken = false;
+      if (odd_sub >= 0) {  // the N-point form of a type-I kind: half the FFT, half the convolution
+        PassArgs B = A;
+        B.sub = odd_sub;
+        B.m /= 2;
+        B.bs_m2 = bluestein_len(B.m, P.real_bytes);
+        taken = take(B);
       }
+      if (!taken) take(A);
     }
   }
   // inside the persistent batch kernel: its mixed-radix tiles (f32, 7-smooth
@@ -3657,6 +3694,8 @@ static void batch_run_plan(pb_batch& B, int i, void* const* buffers, void* ws, c
   }
 }
 
+// Branch mode: one graph whose branches each run a share of the plans with
+// their own pass kernels; forked from and joined back into `s`.
 static void batch_streams(pb_batch* B, int nb) {
   for (int b = (int)B->bstreams.size(); b < nb; ++b) {
     cudaStream_t st;

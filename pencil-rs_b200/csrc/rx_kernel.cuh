@@ -551,8 +551,8 @@ __device__ __forceinline__ void rx_store_c2r(const RxV<R>* rows, const RxArgs& X
 }
 
 // ---- real-to-real kinds, a vector of sequences at a time.  A sequence is a
-// pair p: two real lines 2p, 2p + 1 or the parts of complex line p; kinds IV
-// take one sequence per line or part.
+// pair p: two real lines 2p, 2p + 1 or the parts of complex line p; kinds IV and
+// the odd-N forms of kinds I take one sequence per line or part.
 
 __device__ __forceinline__ Q2 rx_q(float a, float b) { return Q2{make_float2(a, b)}; }
 __device__ __forceinline__ float rx_lane(Q2 q, int w) { return w ? q.v.y : q.v.x; }
@@ -581,7 +581,8 @@ __device__ __forceinline__ typename Vec<R>::Q rx_part(const unsigned char* S, co
   if (A.pre_mode != W_NONE && weight_hit(A.pre_mode, q, A.n)) v = qmul(v, qc<Q>(A.pre_factor));
   return v;
 }
-// Element q of the lines (or parts) that are the sequences of vector g, kinds IV.
+// Element q of the lines (or parts) that are the sequences of vector g, kinds
+// with a sequence per line.
 template <typename R>
 __device__ __forceinline__ typename Vec<R>::Q rx_line(const unsigned char* S, const RxArgs& X, int g, int q) {
   using Q = typename Vec<R>::Q;
@@ -611,7 +612,7 @@ __device__ __forceinline__ RxV<R> rx_dup(typename Cx<R>::T w) {
 // FFT input rows of a real-to-real pass from the staged lines (the
 // definitions of the generic kernel): Makhoul's reordering and pre-twiddle for
 // kinds II / III, the half-length (odd n: zero-padded) form of kinds IV, the
-// symmetric extensions of kinds I.
+// symmetric extensions of kinds I or their odd-N split.
 template <typename R, int SUB, bool BS>
 __device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows, const RxArgs& X) {
   using Q = typename Vec<R>::Q;
@@ -650,6 +651,16 @@ __device__ __forceinline__ void rx_pre_r2r(const unsigned char* S, RxV<R>* rows,
       } else {
         z = {qc<Q>(0.0), qc<Q>(0.0)};
       }
+    } else if constexpr (SUB == S_DST1_ODD || SUB == S_DCT1_ODD) {
+      // c = x_q -+ x_{m-q}, b = (-1)^q (x_q +- x_{m-q}): mr_r2r.cuh
+      constexpr bool DST = SUB == S_DST1_ODD;
+      Q x0 = qc<Q>(0.0), x1 = x0;
+      if (!DST || q > 0) {
+        x0 = rx_line<R>(S, X, g, DST ? q - 1 : q);
+        x1 = rx_line<R>(S, X, g, DST ? m - q - 1 : m - q);
+      }
+      const Q sum = qadd(x0, x1), dif = qsub(x0, x1), bq = DST ? sum : dif;
+      z = {DST ? dif : sum, (q & 1) ? rx_neg(bq) : bq};
     } else if constexpr (SUB == S_DCT1) {
       const int idx = q <= n - 1 ? q : m - q;
       z = {rx_part<R>(S, X, g, 0, idx), rx_part<R>(S, X, g, 1, idx)};
@@ -674,7 +685,7 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
   using Q = typename Vec<R>::Q;
   using C = typename Cx<R>::T;
   const PassArgs& A = X.p;
-  constexpr bool iv4 = SUB == S_DCT4 || SUB == S_DST4;
+  constexpr bool iv4 = r2r_seq_per_line(SUB);
   constexpr int W = Vec<R>::W;
   const int n = A.n, P = X.g.P, lgG = X.g.lgG, total = n << lgG;
   const unsigned mn = fdiv_magic(n);
@@ -685,7 +696,7 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
     int g, k;
     rx_item(it, lgG, n, mn, D.mode == 0, g, k);
     // first destination line of the vector: its values are parts 0 and 1 of W
-    // pairs, or (kinds IV) of W lines or parts
+    // pairs, or (kinds with a sequence per line) of W lines or parts
     const int l = iv4 ? (A.out_complex ? (g * W) >> 1 : g * W) : (A.out_complex ? g * W : 2 * g * W);
     if (l >= D.lines) continue;
     double fs = A.scale;
@@ -710,6 +721,15 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
       const bool neg = SUB == S_DST3 && (k & 1);
       v0 = neg ? rx_neg(z.x) : z.x;
       v1 = neg ? rx_neg(z.y) : z.y;
+    } else if constexpr (SUB == S_DST1_ODD || SUB == S_DCT1_ODD) {
+      const int kk = SUB == S_DST1_ODD ? k + 1 : k;
+      int i = (kk & 1) ? (kk + A.m) >> 1 : kk >> 1;
+      if (SUB == S_DCT1_ODD && i == A.m) i = 0;
+      const RxV<R> z = rows[i * P + g];
+      if (SUB == S_DST1_ODD)
+        v0 = (kk & 1) ? z.x : rx_neg(z.y);
+      else
+        v0 = (kk & 1) ? z.y : z.x;
     } else if constexpr (iv4) {
       if ((n & 1) == 0) {
         const int kk = (k & 1) ? (n - 1 - k) >> 1 : k >> 1;
@@ -771,7 +791,8 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
 }
 
 #define RX_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
-#define RX_SUBS(X) \
+#define RX_SUBS(X)  \
+  X(S_DST1_ODD) X(S_DCT1_ODD) \
   X(S_DCT1) X(S_DCT2) X(S_DCT3) X(S_DCT4) X(S_DST1) X(S_DST2) X(S_DST3) X(S_DST4) X(S_DHT)
 
 // TR: the pass stores transposed (C2C only; the other kinds choose at run

@@ -75,7 +75,7 @@ template std::vector<double> rx_twiddles(const std::vector<int>&, const double*)
 static int lines_x2(const PassArgs& A) {
   if (A.kind == P_C2C) return 2;
   if (A.kind == P_R2C || A.kind == P_C2R) return 4;
-  const bool iv4 = A.sub == S_DCT4 || A.sub == S_DST4;
+  const bool iv4 = r2r_seq_per_line(A.sub);
   if (A.in_complex) return iv4 ? 1 : 2;
   return iv4 ? 2 : 4;
 }
@@ -154,8 +154,8 @@ bool rx_choose(PassArgs& A, int real_bytes, int max_smem, long long max_chunk, l
   for (int s = 0; s < A.nstages; ++s) A.radix[s] = rad[s];
   const int W = real_bytes == 4 ? 2 : 1;
   const int x2 = lines_x2(A);
-  // the type-IV kinds form a pair of lines from two sequences
-  const bool iv4 = A.kind == P_R2R && (A.sub == S_DCT4 || A.sub == S_DST4);
+  // kinds with a sequence per line form a pair of lines from two sequences
+  const bool iv4 = A.kind == P_R2R && r2r_seq_per_line(A.sub);
   const int min_seq = std::max(W, iv4 ? 2 : 1);
   // sequences per tile: a power of two, about 2048 points in f32 and 1024 in
   // f64 (more CTAs per SM beat longer tiles), at least four sequences in f32

@@ -80,3 +80,21 @@ def test_adjoint_weights(make):
     plan.vjp_forward(y, aty)
     lhs, rhs = float(torch.sum((ax.conj() * y).real)), float(torch.sum(x * aty))
     assert abs(lhs - rhs) <= 1e-12 * float(torch.linalg.vector_norm(ax) * torch.linalg.vector_norm(y))
+
+
+@pytest.mark.parametrize("permute", [True, False])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("rb", [4, 8])
+@pytest.mark.parametrize("shape,kinds", [((34, 62, 48), ("DstI",) * 3), ((36, 64, 106), ("DctI",) * 3),
+                                         ((100, 22, 340), ("DstI",) * 3), ((4, 90, 12), ("DctI",) * 3),
+                                         ((10, 384, 6), ("DstI", "DstI", "DctI"))])
+def test_type_one_kinds_with_odd_n(shape, kinds, rb, cplx, permute):
+    """Type-I kinds whose symmetric extension has 2N points, N odd: the N-point
+    form on the compiled and the runtime-radix kernel, Bluestein included."""
+    rng = np.random.default_rng(34)
+    plan = pb.R2rPlan.from_shape(pb.MpiTopology((2, 3)), shape, (3,), kinds, layout=pb.DistributedLayout(permute),
+                                 dtype=CDT[rb] if cplx else RDT[rb])
+    route = po.r2r_route(po.Topology((2, 3)), shape, list(kinds), permute)
+    x = rand_field(rng, shape, (3,), cplx, rb)
+    for d in ("fwd", "inv", "bwd"):
+        check_transform(plan, route, x, 3, rb, cplx, d)
