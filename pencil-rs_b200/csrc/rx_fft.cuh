@@ -211,6 +211,59 @@ struct RxRoots<16> {
     return t[i];
   }
 };
+template <>
+struct RxRoots<17> {
+  static __host__ __device__ constexpr double c(int i) {
+    constexpr double t[17] = {1.0, 0.9324722294043558, 0.7390089172206591, 0.44573835577653825, 0.092268359463302,
+        -0.2736629900720829, -0.6026346363792564, -0.8502171357296141, -0.9829730996839018, -0.9829730996839018,
+        -0.8502171357296141, -0.6026346363792564, -0.2736629900720829, 0.092268359463302, 0.44573835577653825,
+        0.7390089172206591, 0.9324722294043558};
+    return t[i];
+  }
+  static __host__ __device__ constexpr double s(int i) {
+    constexpr double t[17] = {0.0, 0.3612416661871529, 0.6736956436465572, 0.8951632913550623, 0.9957341762950345,
+        0.961825643172819, 0.7980172272802395, 0.5264321628773558, 0.18374951781657034, -0.18374951781657034,
+        -0.5264321628773558, -0.7980172272802395, -0.961825643172819, -0.9957341762950345, -0.8951632913550623,
+        -0.6736956436465572, -0.3612416661871529};
+    return t[i];
+  }
+};
+template <>
+struct RxRoots<19> {
+  static __host__ __device__ constexpr double c(int i) {
+    constexpr double t[19] = {1.0, 0.9458172417006346, 0.7891405093963936, 0.5469481581224269, 0.24548548714079915,
+        -0.08257934547233232, -0.4016954246529695, -0.6772815716257411, -0.8794737512064891, -0.9863613034027223,
+        -0.9863613034027223, -0.8794737512064891, -0.6772815716257411, -0.4016954246529695, -0.08257934547233232,
+        0.24548548714079915, 0.5469481581224269, 0.7891405093963936, 0.9458172417006346};
+    return t[i];
+  }
+  static __host__ __device__ constexpr double s(int i) {
+    constexpr double t[19] = {0.0, 0.3246994692046835, 0.6142127126896678, 0.8371664782625285, 0.9694002659393304,
+        0.9965844930066698, 0.9157733266550574, 0.7357239106731316, 0.47594739303707356, 0.1645945902807339,
+        -0.1645945902807339, -0.47594739303707356, -0.7357239106731316, -0.9157733266550574, -0.9965844930066698,
+        -0.9694002659393304, -0.8371664782625285, -0.6142127126896678, -0.3246994692046835};
+    return t[i];
+  }
+};
+template <>
+struct RxRoots<23> {
+  static __host__ __device__ constexpr double c(int i) {
+    constexpr double t[23] = {1.0, 0.9629172873477992, 0.8544194045464886, 0.6825531432186541, 0.46006503773115215,
+        0.20345601305263378, -0.06824241336467098, -0.33487961217098616, -0.5766803221148672, -0.7757112907044198,
+        -0.917211301505453, -0.9906859460363308, -0.9906859460363308, -0.917211301505453, -0.7757112907044198,
+        -0.5766803221148672, -0.33487961217098616, -0.06824241336467098, 0.20345601305263378, 0.46006503773115215,
+        0.6825531432186541, 0.8544194045464886, 0.9629172873477992};
+    return t[i];
+  }
+  static __host__ __device__ constexpr double s(int i) {
+    constexpr double t[23] = {0.0, 0.2697967711570243, 0.5195839500354336, 0.7308359642781241, 0.8878852184023752,
+        0.9790840876823229, 0.9976687691905392, 0.9422609221188205, 0.816969893010442, 0.6310879443260528,
+        0.39840108984624145, 0.1361666490962466, -0.1361666490962466, -0.39840108984624145, -0.6310879443260528,
+        -0.816969893010442, -0.9422609221188205, -0.9976687691905392, -0.9790840876823229, -0.8878852184023752,
+        -0.7308359642781241, -0.5195839500354336, -0.2697967711570243};
+    return t[i];
+  }
+};
 
 template <typename Q, int RAD> struct VB;
 template <typename Q> struct VB<Q, 2> {
@@ -268,8 +321,44 @@ template <typename Q, int RAD> struct VBOdd {
 template <typename Q> struct VB<Q, 3> : VBOdd<Q, 3> {};
 template <typename Q> struct VB<Q, 5> : VBOdd<Q, 5> {};
 template <typename Q> struct VB<Q, 7> : VBOdd<Q, 7> {};
-template <typename Q> struct VB<Q, 11> : VBOdd<Q, 11> {};
-template <typename Q> struct VB<Q, 13> : VBOdd<Q, 13> {};
+// Butterfly of v, each output handed to emit(r, value) as soon as it is known:
+// the outputs of the larger odd radices are not held next to their inputs.
+template <typename Q, int RAD, typename F>
+__device__ __forceinline__ void vb_emit(VC<Q>* v, F&& emit) {
+  if constexpr (RAD == 11 || RAD == 13 || RAD > 16) {
+    constexpr int H = (RAD - 1) / 2;
+    VC<Q> s0 = v[0];
+#pragma unroll
+    for (int p = 1; p <= H; ++p) {
+      const VC<Q> t = v[p];
+      v[p] = vadd(t, v[RAD - p]);
+      v[RAD - p] = vsub(t, v[RAD - p]);
+      s0 = vadd(s0, v[p]);
+    }
+    emit(0, s0);
+#pragma unroll
+    for (int q = 1; q <= H; ++q) {
+      VC<Q> A = v[0], B;
+#pragma unroll
+      for (int p = 1; p <= H; ++p) {
+        const int i = (p * q) % RAD;
+        const Q c = qc<Q>(RxRoots<RAD>::c(i)), s = qc<Q>(RxRoots<RAD>::s(i));
+        A = {qfma(v[p].x, c, A.x), qfma(v[p].y, c, A.y)};
+        if (p == 1)
+          B = {qmul(v[RAD - 1].x, s), qmul(v[RAD - 1].y, s)};
+        else
+          B = {qfma(v[RAD - p].x, s, B.x), qfma(v[RAD - p].y, s, B.y)};
+      }
+      emit(q, vaddr(A, B));
+      emit(RAD - q, vsubr(A, B));
+    }
+  } else {
+    VB<Q, RAD>::run(v);
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) emit(r, v[r]);
+  }
+}
+
 template <typename Q, int R1, int R2> struct VBComp {
   static __device__ __forceinline__ void run(VC<Q>* v) {
     constexpr int NN = R1 * R2;

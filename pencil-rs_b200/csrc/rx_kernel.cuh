@@ -45,6 +45,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "pb_device.cuh"
 #include "pb_launch.cuh"
 #include "rx_fft.cuh"
@@ -193,6 +195,9 @@ __device__ __forceinline__ constexpr int rx_lines_per_vec() {
   return Vec<R>::W * (KIND == P_C2C ? 1 : 2);
 }
 
+// Row of element i: padded by one row after every `pad` (magic mp).
+__device__ __forceinline__ int rx_row(int i, int pad, unsigned mp) { return pad ? i + (int)fdiv(i, pad, mp) : i; }
+
 // Stage 0 (no twiddles) from the staged lines.
 template <typename R, int KIND, int RAD>
 __device__ __forceinline__ void rx_first(const unsigned char* S, RxV<R>* out, const RxArgs& X) {
@@ -214,10 +219,8 @@ __device__ __forceinline__ void rx_first(const unsigned char* S, RxV<R>* out, co
 #pragma unroll
       for (int r = 1; r < RAD; ++r) v[r] = rx_fetch_at<R, KIND>(S, base, sl, b0 + r * st);
     }
-    VB<Q, RAD>::run(v);
-    RxV<R>* o = out + jb * RAD * P + g;
-#pragma unroll
-    for (int r = 0; r < RAD; ++r) o[r * P] = v[r];
+    RxV<R>* o = out + jb * (RAD + (X.g.pad ? 1 : 0)) * P + g;
+    vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r * P] = x; });
   }
 }
 
@@ -253,17 +256,19 @@ __device__ __forceinline__ VC<Q> rx_ldg(const VC<Q>* p) {
   *reinterpret_cast<float4*>(&r) = f;
   return r;
 }
+// ip, op: the padding of the rows read and written.
 template <typename R, int RAD, int MODE>
 __device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int NS, const RxV<R>* tw,
-                                       const RxV<R>* mul, int lim) {
+                                       const RxV<R>* mul, int lim, int ip, int op) {
   using Q = typename Vec<R>::Q;
   const int len = X.g.len, NB = len / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
-  const int rs = NB * P, ws = NS * P;
-  const unsigned mNS = fdiv_magic(NS);
+  const unsigned mNS = fdiv_magic(NS), mpad = X.g.pad ? fdiv_magic(X.g.pad) : 0;
+  // NB (after stage 0) and NS (of later stages) are multiples of the padding
+  const int rs = (NB + (ip ? NB / ip : 0)) * P, ws = (NS + (op && NS > 1 ? NS / op : 0)) * P;
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
     const int g = it & ((1 << lgG) - 1), jb = it >> lgG;
     const int k = MODE == kMidMul ? 0 : jb - (int)fdiv(jb, NS, mNS) * NS;
-    const RxV<R>* p = in + jb * P + g;
+    const RxV<R>* p = in + rx_row(jb, ip, mpad) * P + g;
     RxV<R> v[RAD];
     if constexpr (MODE == kMidMul) {
 #pragma unroll
@@ -280,17 +285,14 @@ __device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxAr
         for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NS]);
       }
     }
-    VB<Q, RAD>::run(v);
     if constexpr (MODE == kMidOut) {
-#pragma unroll
-      for (int r = 0; r < RAD; ++r) {
+      vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) {
         const int i = (jb - k) * RAD + k + r * NS, o = i == 0 ? 0 : len - i;
-        if (o < lim) out[o * P + g] = vtw(v[r], rx_ldg(mul + o));
-      }
+        if (o < lim) out[o * P + g] = vtw(x, rx_ldg(mul + o));
+      });
     } else {
-      RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
-#pragma unroll
-      for (int r = 0; r < RAD; ++r) o[r * ws] = v[r];
+      RxV<R>* o = out + rx_row((jb - k) * RAD + k, op, mpad) * P + g;
+      vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r * ws] = x; });
     }
   }
 }
@@ -300,16 +302,16 @@ __device__ __forceinline__ void rx_mid(const RxV<R>* in, RxV<R>* out, const RxAr
 // sits in registers.  `roots` are the RAD-th roots.
 template <typename R>
 __device__ __forceinline__ void rx_mid_prime(const RxV<R>* in, RxV<R>* out, const RxArgs& X, int RAD, int NS,
-                                             const RxV<R>* tw, const RxV<R>* roots) {
+                                             const RxV<R>* tw, const RxV<R>* roots, int ip, int op) {
   const int NB = X.g.len / RAD, lgG = X.g.lgG, P = X.g.P;
   const int H = (RAD - 1) / 2, total = (NB * (H + 1)) << lgG;
-  const int rs = NB * P, ws = NS * P;
-  const unsigned mNS = fdiv_magic(NS), mNB = fdiv_magic(NB);
+  const unsigned mNS = fdiv_magic(NS), mNB = fdiv_magic(NB), mpad = X.g.pad ? fdiv_magic(X.g.pad) : 0;
+  const int rs = (NB + (ip ? NB / ip : 0)) * P, ws = (NS + (op && NS > 1 ? NS / op : 0)) * P;
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
     const int g = it & ((1 << lgG) - 1), b = it >> lgG;
     const int h = (int)fdiv(b, NB, mNB), jb = b - h * NB;
     const int k = jb - (int)fdiv(jb, NS, mNS) * NS;
-    const RxV<R>* p = in + jb * P + g;
+    const RxV<R>* p = in + rx_row(jb, ip, mpad) * P + g;
     const RxV<R> v0 = p[0];
     RxV<R> a = v0, c = {qc<typename Vec<R>::Q>(0.0), qc<typename Vec<R>::Q>(0.0)};
     int idx = 0;
@@ -326,7 +328,7 @@ __device__ __forceinline__ void rx_mid_prime(const RxV<R>* in, RxV<R>* out, cons
       a = {qfma(s.x, t.x, a.x), qfma(s.y, t.x, a.y)};
       c = {qfma(d.x, t.y, c.x), qfma(d.y, t.y, c.y)};
     }
-    RxV<R>* o = out + ((jb - k) * RAD + k) * P + g;
+    RxV<R>* o = out + rx_row((jb - k) * RAD + k, op, mpad) * P + g;
     // sum over d * (-i sin): a + i c with c carrying -sin
     if (h == 0) {
       o[0] = a;
@@ -404,8 +406,8 @@ __device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const
   using Q = typename Vec<R>::Q;
   using C = typename Cx<R>::T;
   const int NB = X.p.m / RAD, lgG = X.g.lgG, P = X.g.P, total = NB << lgG;
-  const int rs = NB * P;
-  const unsigned mNB = fdiv_magic(NB);
+  const int pad = X.g.pad, rs = (NB + (pad ? NB / pad : 0)) * P;
+  const unsigned mNB = fdiv_magic(NB), mpad = pad ? fdiv_magic(pad) : 0;
   const Q sc = qc<Q>(X.p.scale);
   C* out = reinterpret_cast<C*>(X.p.out);
   for (int it = threadIdx.x; it < total; it += blockDim.x) {
@@ -413,31 +415,29 @@ __device__ __forceinline__ void rx_last(const RxV<R>* in, const RxArgs& X, const
     rx_item(it, lgG, NB, mNB, TR, g, jb);
     const int l = g * Vec<R>::W;
     if (l >= D.lines) continue;
-    const RxV<R>* p = in + jb * P + g;
+    const RxV<R>* p = in + rx_row(jb, pad, mpad) * P + g;
     RxV<R> v[RAD];
 #pragma unroll
     for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
     const RxV<R>* t = tw + jb;
 #pragma unroll
     for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NB]);
-    VB<Q, RAD>::run(v);
     if (!TR && D.mode == 1) {
       C* o = out + D.dst0 + (long long)l * D.dstb + jb;
       const bool two = sizeof(R) == 4 && l + 1 < D.lines;
-#pragma unroll
-      for (int r = 0; r < RAD; ++r) {
-        const RxV<R> w = {qmul(v[r].x, sc), qmul(v[r].y, sc)};
+      vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) {
+        const RxV<R> w = {qmul(x.x, sc), qmul(x.y, sc)};
         if constexpr (sizeof(R) == 4) {
           o[r * NB] = make_float2(w.x.v.x, w.y.v.x);
           if (two) o[D.dstb + r * NB] = make_float2(w.x.v.y, w.y.v.y);
         } else {
           o[r * NB] = make_double2(w.x, w.y);
         }
-      }
+      });
     } else {
-#pragma unroll
-      for (int r = 0; r < RAD; ++r)
-        rx_put_c2c<R>(out, D, jb + r * NB, l, RxV<R>{qmul(v[r].x, sc), qmul(v[r].y, sc)});
+      vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) {
+        rx_put_c2c<R>(out, D, jb + r * NB, l, RxV<R>{qmul(x.x, sc), qmul(x.y, sc)});
+      });
     }
   }
 }
@@ -790,7 +790,9 @@ __device__ __forceinline__ void rx_post_r2r(const RxV<R>* rows, const RxArgs& X,
   }
 }
 
-#define RX_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+// radices of the convolution lengths, and of the other lengths
+#define RX_RADICES_BS(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(15) X(16)
+#define RX_RADICES(X) RX_RADICES_BS(X) X(11) X(13) X(17) X(19) X(23)
 #define RX_SUBS(X)  \
   X(S_DST1_ODD) X(S_DCT1_ODD) \
   X(S_DCT1) X(S_DCT2) X(S_DCT3) X(S_DCT4) X(S_DST1) X(S_DST2) X(S_DST3) X(S_DST4) X(S_DHT)
@@ -913,8 +915,8 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
         const int lim = f ? g.len : A.m;
         switch (A.radix[0]) {
 #define X_(r) \
-  case r: rx_mid<R, r, kMidMul>(in, out, X, 1, nullptr, mul, lim); break;
-          RX_RADICES(X_)
+  case r: rx_mid<R, r, kMidMul>(in, out, X, 1, nullptr, mul, lim, 0, g.pad); break;
+          RX_RADICES_BS(X_)
 #undef X_
         }
         swap();
@@ -925,15 +927,15 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
           if (f == 1 && s == A.nstages - 1) {
             switch (rad) {
 #define X_(r) \
-  case r: rx_mid<R, r, kMidOut>(in, out, X, NS, t, chirp, A.m); break;
-              RX_RADICES(X_)
+  case r: rx_mid<R, r, kMidOut>(in, out, X, NS, t, chirp, A.m, g.pad, 0); break;
+              RX_RADICES_BS(X_)
 #undef X_
             }
           } else {
             switch (rad) {
 #define X_(r) \
-  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0); break;
-              RX_RADICES(X_)
+  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0, g.pad, s + 1 < A.nstages ? g.pad : 0); break;
+              RX_RADICES_BS(X_)
 #undef X_
             }
           }
@@ -945,12 +947,15 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
       for (int s = s0; s < last; ++s) {
         const int rad = A.radix[s];
         const V* t = tw + g.twoff[s];
+        // the stages' rows are padded; the rows formed before stage 0 and the
+        // finished ones are not
+        const int ip = s > 0 ? g.pad : 0, op = s + 1 < A.nstages ? g.pad : 0;
         switch (rad) {
 #define X_(r) \
-  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0); break;
+  case r: rx_mid<R, r, kMidPlain>(in, out, X, NS, t, nullptr, 0, ip, op); break;
           RX_RADICES(X_)
 #undef X_
-          default: rx_mid_prime<R>(in, out, X, rad, NS, t, t + (s > 0 ? (rad - 1) * NS : 0)); break;
+          default: rx_mid_prime<R>(in, out, X, rad, NS, t, t + (s > 0 ? (rad - 1) * NS : 0), ip, op); break;
         }
         swap();
         NS *= rad;
@@ -988,6 +993,172 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
       rx_stage<R, KIND>(S, X, tn);
       rx_cp_commit();
     }
+  }
+}
+
+// ---- in place: long C2C and R2C lines (g.ip), one vector per row, a butterfly
+// per thread and stage.  A stage's rows are all read before any is written, so
+// one row buffer serves and two CTAs fit on an SM; the lines go from memory
+// into registers, and the other CTA computes meanwhile.
+
+template <typename R, int KIND, int RAD>
+__device__ __forceinline__ void rx_ip_first(const TileAddr& ta, RxV<R>* rows, const RxArgs& X) {
+  using Q = typename Vec<R>::Q;
+  using E = std::conditional_t<KIND == P_C2C, typename Cx<R>::T, R>;
+  const PassArgs& A = X.p;
+  const int m = A.m, NB = m / RAD, jb = threadIdx.x;
+  if (jb >= NB) return;
+  constexpr int NL = Vec<R>::W * (KIND == P_C2C ? 1 : 2);  // lines of a vector
+  const E* in = reinterpret_cast<const E*>(A.in) + ta.src0;
+  const long long sq = A.src_k_contig ? 1 : ta.srcq, lb = ta.srcb;
+  const int lines = ta.lines;
+  RxV<R> v[RAD];
+#pragma unroll
+  for (int r = 0; r < RAD; ++r) {
+    // element jb + r*NB, or its mirror m - element when inverse
+    const int q = jb + r * NB;
+    const E* p = in + (long long)((A.inv && q != 0) ? m - q : q) * sq;
+    E x[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      if (l < lines)
+        x[l] = p[l * lb];
+      else
+        memset(&x[l], 0, sizeof(E));
+    }
+    if constexpr (KIND == P_C2C) {
+      if constexpr (sizeof(R) == 4)
+        v[r] = rx_pack(x[0].x, x[0].y, x[1].x, x[1].y);
+      else
+        v[r] = RxV<R>{x[0].x, x[0].y};
+    } else {
+      if constexpr (sizeof(R) == 4)
+        v[r] = rx_pack(x[0], x[1], x[2], x[3]);
+      else
+        v[r] = RxV<R>{x[0], x[1]};
+    }
+  }
+  RxV<R>* o = rows + jb * (RAD + (X.g.pad ? 1 : 0));
+  vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r] = x; });
+}
+
+template <typename R, int RAD>
+__device__ __forceinline__ void rx_ip_mid(RxV<R>* rows, const RxArgs& X, int NS, const RxV<R>* tw, int op) {
+  using Q = typename Vec<R>::Q;
+  const int NB = X.g.len / RAD, pad = X.g.pad;
+  const bool act = (int)threadIdx.x < NB;
+  const int jb = act ? threadIdx.x : NB - 1;  // idle threads read along, and write nothing
+  const unsigned mpad = pad ? fdiv_magic(pad) : 0;
+  const int rs = NB + (pad ? NB / pad : 0), ws = NS + (op ? NS / op : 0);
+  const int k = jb - (int)fdiv(jb, NS, fdiv_magic(NS)) * NS;
+  RxV<R> v[RAD];
+  const RxV<R>* p = rows + rx_row(jb, pad, mpad);
+#pragma unroll
+  for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
+  const RxV<R>* t = tw + k;
+#pragma unroll
+  for (int r = 1; r < RAD; ++r) v[r] = vtw(v[r], t[(r - 1) * NS]);
+  // the block barrier, its own in each radix's code: a shared one would keep the
+  // values of every radix alive across it
+  asm volatile("bar.sync 0; // radix %0" ::"n"(RAD) : "memory");
+  if (act) {
+    RxV<R>* o = rows + rx_row((jb - k) * RAD + k, op, mpad);
+    vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r * ws] = x; });
+  }
+}
+
+template <typename R, int KIND, bool TR>
+__global__ void __launch_bounds__(kRxMaxThreads, 1) rx_inplace_kernel(const __grid_constant__ RxArgs X) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using V = RxV<R>;
+  const PassArgs& A = X.p;
+  const RxGeom& g = X.g;
+  if (pb_rejected(A.gate)) return;
+  long long tile = blockIdx.x;
+  const long long step = gridDim.x, end = A.ntiles;
+  if (tile >= end) return;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  V* rows = reinterpret_cast<V*>(smem);
+  V* W = reinterpret_cast<V*>(smem + g.off_tw);
+  TileAddr* desc = reinterpret_cast<TileAddr*>(smem + g.off_desc);  // tiles i, i+1
+  PieceAddr* prow = reinterpret_cast<PieceAddr*>(desc + 3);         // pieces of tiles i, i+1
+  const V* Wg = reinterpret_cast<const V*>(A.twiddle);
+  const V* tw = g.tw_smem ? W : Wg;
+  const TileAddr* tiles = reinterpret_cast<const TileAddr*>(A.tile_tab);
+  const PieceAddr* pieces = reinterpret_cast<const PieceAddr*>(A.piece_tab);
+  const int mode = KIND == P_C2C && TR ? 0 : A.dst_k_contig;
+  const int np = mode == 1 ? 0 : A.npieces;
+  RxDst D;
+  D.mode = mode;
+  D.np = np;
+  D.nout = A.n_out;
+  D.mnout = fdiv_magic(A.n_out);
+  const long long pst = np > 0 ? (long long)A.n_out * tid / np : 0;
+  if (tid == 0) desc[0] = load_tile(tiles, tile);
+  if (tid < np) prow[tid] = pieces[tile * np + tid];
+  for (int i = tid; i < g.tw_smem; i += nt) W[i] = Wg[i];
+  pb_dependency_wait();  // the tables above belong to the plan; the data is read from here on
+
+  for (int par = 0;; par ^= 1, tile += step) {
+    rx_cp_wait();
+    PieceAddr* pr = prow + par * kRxMaxPieces;
+    if (tid < np) {
+      PieceAddr pa = pr[tid];
+      pa.rowbase -= mode == 0 ? pst * pa.stride : pst;
+      pr[tid] = pa;
+    }
+    __syncthreads();  // descriptor, pieces and twiddles in place; the previous tile's rows are free
+    const TileAddr& ta = desc[par];
+    D.dst0 = ta.dst0;
+    D.dstb = ta.dstb;
+    D.lines = ta.lines;
+    D.prow = pr;
+    const bool has_next = tile + step < end;
+    if (has_next) {
+      if (tid == 0) {
+        char* d = reinterpret_cast<char*>(desc + (par ^ 1));
+        const char* t = reinterpret_cast<const char*>(tiles + tile + step);
+        rx_cp_async<16>(d, t);
+        rx_cp_async<16>(d + 16, t + 16);
+      }
+      if (tid < np) rx_cp_async<16>(prow + (par ^ 1) * kRxMaxPieces + tid, pieces + (tile + step) * np + tid);
+      rx_cp_commit();
+    } else {
+      pb_allow_successor();
+    }
+    switch (A.radix[0]) {
+#define X_(r) \
+  case r: rx_ip_first<R, KIND, r>(ta, rows, X); break;
+      RX_RADICES(X_)
+#undef X_
+    }
+    __syncthreads();
+    int NS = A.radix[0];
+    const int last = KIND == P_C2C ? A.nstages - 1 : A.nstages;
+    for (int s = 1; s < last; ++s) {
+      const V* t = tw + g.twoff[s];
+      const int op = s + 1 < A.nstages ? g.pad : 0;
+      switch (A.radix[s]) {
+#define X_(r) \
+  case r: rx_ip_mid<R, r>(rows, X, NS, t, op); break;
+        RX_RADICES(X_)
+#undef X_
+      }
+      __syncthreads();
+      NS *= A.radix[s];
+    }
+    if constexpr (KIND == P_C2C) {
+      const V* t = tw + g.twoff[last];
+      switch (A.radix[last]) {
+#define X_(r) \
+  case r: rx_last<R, r, TR>(rows, X, t, D); break;
+        RX_RADICES(X_)
+#undef X_
+      }
+    } else {
+      rx_store_r2c<R>(rows, X, D);
+    }
+    if (!has_next) break;
   }
 }
 

@@ -9,15 +9,20 @@ template <int KIND>
 using RxFn = void (*)(const RxArgs);
 
 template <typename R>
-static RxFn<RX_KIND> rx_pick(const PassArgs& A) {
+static RxFn<RX_KIND> rx_pick(const RxArgs& X) {
 #if RX_BS
-  (void)A;
+  (void)X;
   return rx_kernel<R, RX_KIND, false, true>;
 #else
-  if constexpr (RX_KIND == P_C2C)
-    return A.dst_k_contig == 0 ? rx_kernel<R, RX_KIND, true, false> : rx_kernel<R, RX_KIND, false, false>;
-  else
+  if constexpr (RX_KIND == P_C2C) {
+    if (X.p.dst_k_contig == 0)
+      return X.g.ip ? rx_inplace_kernel<R, RX_KIND, true> : rx_kernel<R, RX_KIND, true, false>;
+    return X.g.ip ? rx_inplace_kernel<R, RX_KIND, false> : rx_kernel<R, RX_KIND, false, false>;
+  } else if constexpr (RX_KIND == P_R2C) {
+    return X.g.ip ? rx_inplace_kernel<R, RX_KIND, false> : rx_kernel<R, RX_KIND, false, false>;
+  } else {
     return rx_kernel<R, RX_KIND, false, false>;
+  }
 #endif
 }
 
@@ -27,6 +32,13 @@ static cudaError_t rx_allow_smem(const RxArgs& X) {
 #if RX_BS
   return pb_allow_smem<rx_kernel<R, RX_KIND, false, true>>(X.g.max_smem);
 #else
+  if constexpr (RX_KIND == P_C2C || RX_KIND == P_R2C) {
+    if (X.g.ip) {
+      if constexpr (RX_KIND == P_C2C)
+        if (X.p.dst_k_contig == 0) return pb_allow_smem<rx_inplace_kernel<R, RX_KIND, true>>(X.g.max_smem);
+      return pb_allow_smem<rx_inplace_kernel<R, RX_KIND, false>>(X.g.max_smem);
+    }
+  }
   if constexpr (RX_KIND == P_C2C)
     if (X.p.dst_k_contig == 0) return pb_allow_smem<rx_kernel<R, RX_KIND, true, false>>(X.g.max_smem);
   return pb_allow_smem<rx_kernel<R, RX_KIND, false, false>>(X.g.max_smem);
@@ -40,7 +52,7 @@ int rx_occupancy_kind(const RxArgs& X, int real_bytes);
 
 template <>
 cudaError_t rx_launch_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes, int grid, cudaStream_t stream) {
-  const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
+  const auto kern = real_bytes == 4 ? rx_pick<float>(X) : rx_pick<double>(X);
   const cudaError_t err = real_bytes == 4 ? rx_allow_smem<float>(X) : rx_allow_smem<double>(X);
   if (err != cudaSuccess) return err;
   return pb_launch<RxArgs>(kern, grid, X.g.threads, X.g.smem, stream, X);
@@ -48,7 +60,7 @@ cudaError_t rx_launch_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes, int 
 
 template <>
 int rx_occupancy_kind<RX_KIND, RX_BS>(const RxArgs& X, int real_bytes) {
-  const auto kern = real_bytes == 4 ? rx_pick<float>(X.p) : rx_pick<double>(X.p);
+  const auto kern = real_bytes == 4 ? rx_pick<float>(X) : rx_pick<double>(X);
   int blocks = 0;
   if ((real_bytes == 4 ? rx_allow_smem<float>(X) : rx_allow_smem<double>(X)) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, X.g.threads, X.g.smem) != cudaSuccess)

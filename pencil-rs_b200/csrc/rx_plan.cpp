@@ -71,7 +71,7 @@ template std::vector<float> rx_twiddles(const std::vector<int>&, const float*);
 template std::vector<double> rx_twiddles(const std::vector<int>&, const double*);
 
 // Real lines per FFT sequence, doubled: C2C 2 (one line), line pairs 4, the
-// type-IV kinds 2 (real data) or 1 (complex data: a sequence per component).
+// kinds with a sequence per line 2 (real data) or 1 (complex data: a sequence per component).
 static int lines_x2(const PassArgs& A) {
   if (A.kind == P_C2C) return 2;
   if (A.kind == P_R2C || A.kind == P_C2R) return 4;
@@ -93,8 +93,13 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
   // contiguous in the destination from tiles of more than four vectors) hit
   // distinct banks; the other stores read whole rows and need none
   g->P = (A.dst_k_contig != 0 && G > 4) ? G + 1 : G;
-  g->bufv = g->len * g->P;
   g->pre = (A.kind == P_R2R || A.bs_m2 || A.radix[0] > kRxRegRadix) ? 1 : 0;
+  // stage 0 writes rows at multiples of its radix: with an even one and less
+  // than eight vectors to a row, one row of padding after every radix[0] rows
+  // puts them on distinct banks (4096 = 16*16*16 points: half of the
+  // wavefronts were conflicts)
+  g->pad = (A.radix[0] % 2 == 0 && G < 8 && A.nstages > 1) ? A.radix[0] : 0;
+  g->bufv = (g->len + (g->pad ? g->len / g->pad : 0)) * g->P;
   long long tw = 0, ns = 1;
   for (int s = 0; s < A.nstages; ++s) {
     g->twoff[s] = (int)tw;
@@ -139,7 +144,25 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
     g->smem = (int)b;
     return true;
   };
-  const bool ok = fits(true, false) || fits(false, false) || fits(true, true) || fits(false, true);
+  bool ok = fits(true, false) || fits(false, false) || fits(true, true) || fits(false, true);
+  // Long lines, whose tile of the fewest sequences leaves one CTA per SM: C2C
+  // and R2C passes run in place, one butterfly per thread and stage, so that
+  // two CTAs fit and one loads while the other computes.
+  int items = 0;
+  for (int s = 0; s < A.nstages; ++s) items = std::max(items, g->len / A.radix[s]);
+  if ((A.kind == P_C2C || A.kind == P_R2C) && !g->pre && A.nstages > 1 && G == 1 && items <= kRxMaxThreads &&
+      (!ok || 2 * (g->smem + 1024) > max_smem)) {
+    const int half = (max_smem - 1024) / 2;
+    const int room = half - buf_bytes - tail;
+    g->ip = 1;
+    g->alias = 0;
+    g->tw_smem = tw_bytes <= room ? (int)tw : 0;
+    g->off_tw = buf_bytes;
+    g->off_stage = g->off_desc = buf_bytes + g->tw_smem * 16;
+    g->smem = g->off_desc + tail;
+    g->threads = std::max(128, (items + 31) / 32 * 32);
+    return g->smem <= max_smem;
+  }
   if (!ok) return false;
   const long long elems = (long long)nseq * g->len;
   g->threads = elems > 6 * 1024 / (3 - W) ? 512 : elems > 2600 / (3 - W) ? 256 : 128;

@@ -15,7 +15,7 @@ constexpr int kRxMaxThreads = 512;
 constexpr int kRxMaxPieces = 64;
 // largest radix with a butterfly in registers; larger primes take the
 // direct-sum stage
-constexpr int kRxRegRadix = 16;
+constexpr int kRxRegRadix = 23;
 
 // Tile geometry of one pass, a function of its PassArgs (rx_geometry).  Shared
 // memory: two row buffers (row i of a buffer is element i of every sequence:
@@ -30,6 +30,8 @@ struct RxGeom {
   int pre;       // 1: a pass over the staged lines forms the FFT input rows first
   int tw_smem;   // twiddle vectors held in shared memory (0: read from global memory)
   int alias;     // 1: the staging area is the second row buffer (no prefetch overlap)
+  int ip;        // 1: stages in place in one row buffer, lines read straight into registers
+  int pad;       // rows written by a stage are padded by one after every `pad` (0: none)
   int sl, sq;    // staging strides of a line and of an element, in elements
   int off_tw, off_stage, off_desc;  // byte offsets in shared memory
   int smem;      // bytes
