@@ -25,9 +25,17 @@ _REAL = {torch.float32: (0, False), torch.float64: (1, False), torch.complex64: 
          torch.complex128: (1, True)}
 
 
+# the current device's current stream as a raw handle: torch.cuda.current_stream
+# builds a Stream object, 3.3 us of the 14 us of host time of a three-pass call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream) -> C.c_void_p:
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    if _raw_stream is None:
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_raw_stream(torch.cuda.current_device()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
