@@ -7,15 +7,24 @@
 // convolution of length N = A.bs_m2 (the smallest of kBluesteinLengths
 // >= 2m - 1).  One tile of
 // NSEQ lines runs, without leaving shared memory:
-//   * the stage-0 load of the lines times the chirp, zero past m (registers);
-//   * the forward N-point Stockham FFT (mr_stage0, mr_stages_upto);
-//   * the product with the transform of the periodic conjugate chirp
-//     (A.bs_kernel, with the 1/N of the inverse folded in);
-//   * the inverse N-point FFT, its stage 0 fed from shared memory;
+//   * the stage-0 load of the lines, zero past m (registers, one tile ahead:
+//     nothing is computed from them until their tile starts, so that they
+//     overlap the tile before);
+//   * the product with the chirp and the forward N-point Stockham FFT
+//     (mr_stage0, mr_stages_upto);
+//   * the inverse N-point FFT, its stage 0 fed from shared memory times the
+//     transform of the periodic conjugate chirp (A.bs_kernel, with the 1/N of
+//     the inverse folded in);
 //   * the post-chirp and the store (C2C outputs k < m, C2R the two real
 //     lines, R2C the split half spectra of the pair).
-// The generic kernel's FFT core (pass_kernel.cu, fft_run) computes the same
-// convolution for the real-to-real kinds and for longer lines.
+// What bounds it: barriers and latency.  With the chirp product at the load
+// (which waits for the next tile's data) and the kernel product in a pass of
+// its own, 257-point passes ran at 1.07 (C2C f32) and 0.95 TB/s (R2C f32)
+// instead of 1.13 and 1.11, 127-point f64 ones at 1.32 (transposed) and 1.35
+// (direct) instead of 1.43 and 1.58.
+// The runtime-radix kernel (rx_kernel.cuh) computes the same convolution for the
+// real-to-real kinds and for longer lines, the generic kernel's FFT core
+// (pass_kernel.cu, fft_run) for the layouts that neither takes.
 #pragma once
 
 #include "mr_kernel.cuh"
@@ -38,7 +47,6 @@ __device__ __forceinline__ void mr_load_bs(typename Cx<R>::T (&v)[MRGeom<R, N>::
   const R zero = R(0);
   const int L = ta.lines;
   const int m = A.m;
-  const C* __restrict__ chirp = reinterpret_cast<const C*>(A.bs_chirp);
 #pragma unroll
   for (int u = 0; u < G::U0; ++u) {
     const int b = threadIdx.x + u * MR_THREADS;
@@ -53,7 +61,7 @@ __device__ __forceinline__ void mr_load_bs(typename Cx<R>::T (&v)[MRGeom<R, N>::
 #pragma unroll
       for (int r = 0; r < R0; ++r) {
         const int q = jb + r * NB;
-        v[u][r] = (ok && q < m) ? cmul(in[base + q * sq], chirp[q]) : mk<C, R>(zero, zero);
+        v[u][r] = (ok && q < m) ? in[base + q * sq] : mk<C, R>(zero, zero);
       }
     } else if (A.kind == P_R2C) {  // real lines 2s, 2s+1 as x + iy
       const R* __restrict__ in = reinterpret_cast<const R*>(A.in);
@@ -63,8 +71,7 @@ __device__ __forceinline__ void mr_load_bs(typename Cx<R>::T (&v)[MRGeom<R, N>::
 #pragma unroll
       for (int r = 0; r < R0; ++r) {
         const int q = jb + r * NB;
-        const C z = mk<C, R>((ok0 && q < m) ? in[b0 + q * sq] : zero, (ok1 && q < m) ? in[b1 + q * sq] : zero);
-        v[u][r] = q < m ? cmul(z, chirp[q]) : mk<C, R>(zero, zero);
+        v[u][r] = mk<C, R>((ok0 && q < m) ? in[b0 + q * sq] : zero, (ok1 && q < m) ? in[b1 + q * sq] : zero);
       }
     } else {  // C2R: the Hermitian extensions of half spectra 2s, 2s+1 as X + iY
       const C* __restrict__ in = reinterpret_cast<const C*>(A.in);
@@ -94,7 +101,7 @@ __device__ __forceinline__ void mr_load_bs(typename Cx<R>::T (&v)[MRGeom<R, N>::
           Y.y = zero;
         }
         const R w = (weighted && !edge) ? w_in : R(1);
-        v[u][r] = cmul(mk<C, R>((X.x - Y.y) * w, (X.y + Y.x) * w), chirp[q]);
+        v[u][r] = mk<C, R>((X.x - Y.y) * w, (X.y + Y.x) * w);
       }
     }
   }
@@ -113,7 +120,18 @@ __device__ __forceinline__ void mr_tile_bs(const PassArgs& A, const TileAddr& ta
   const int tid = threadIdx.x;
   const int m = A.m;
   const R zero = R(0);
-  // forward N-point FFT of the chirped lines
+  // forward N-point FFT of the lines times the chirp (the inputs past m are zero)
+  const C* __restrict__ chirp = reinterpret_cast<const C*>(A.bs_chirp);
+#pragma unroll
+  for (int u = 0; u < G::U0; ++u) {
+    const int b = threadIdx.x + u * MR_THREADS;
+    const int jb = SX ? b / G::NSEQ : b % NB;
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      const int q = jb + r * NB;
+      if (q < m) v[u][r] = cmul(v[u][r], chirp[q]);
+    }
+  }
   mr_stage0<R, N, false, SX>(v, b0);
   if (tid < npieces) prow[tid] = my_piece;
   __syncthreads();
@@ -132,15 +150,9 @@ __device__ __forceinline__ void mr_tile_bs(const PassArgs& A, const TileAddr& ta
   }
   mr_stages_upto<R, N, false, 1, G::NST>(b0, b1, W);
   C* F = ((G::NST - 1) % 2 == 0) ? b0 : b1;
-  // product with the convolution kernel
+  // inverse N-point FFT: stage-0 inputs from shared memory, times the
+  // convolution kernel
   const C* __restrict__ ker = reinterpret_cast<const C*>(A.bs_kernel);
-  for (int i = tid; i < G::NSEQ * N; i += MR_THREADS) {
-    const int s = i / N, k = i - (i / N) * N;
-    C* p = F + s * G::SEQ + G::pad(k);
-    *p = cmul(*p, ker[k]);
-  }
-  __syncthreads();
-  // inverse N-point FFT: stage-0 inputs from shared memory
 #pragma unroll
   for (int u = 0; u < G::U0; ++u) {
     const int b = threadIdx.x + u * MR_THREADS;
@@ -148,7 +160,8 @@ __device__ __forceinline__ void mr_tile_bs(const PassArgs& A, const TileAddr& ta
     const int jb = b - s * NB;
     const bool live = (G::B0 % MR_THREADS == 0) || b < G::B0;
 #pragma unroll
-    for (int r = 0; r < R0; ++r) v[u][r] = live ? F[s * G::SEQ + G::pad(jb + r * NB)] : mk<C, R>(zero, zero);
+    for (int r = 0; r < R0; ++r)
+      v[u][r] = live ? cmul(F[s * G::SEQ + G::pad(jb + r * NB)], ker[jb + r * NB]) : mk<C, R>(zero, zero);
   }
   __syncthreads();  // F may be b0, which stage 0 writes
   mr_stage0<R, N, true>(v, b0);
@@ -158,7 +171,6 @@ __device__ __forceinline__ void mr_tile_bs(const PassArgs& A, const TileAddr& ta
   // post-chirp and store: C2C outputs k < m; C2R the real and imaginary parts
   // of z_q (q < m) as lines 2p, 2p+1; R2C the split half spectra (k <= m/2)
   // of the pair's Z
-  const C* __restrict__ chirp = reinterpret_cast<const C*>(A.bs_chirp);
   const R sc = R(A.scale);
   const int L = ta.lines;
   const bool direct = A.dst_k_contig != 0;  // line-major order for both direct stores
