@@ -996,8 +996,7 @@ __global__ void __launch_bounds__(kRxMaxThreads, 1) rx_kernel(const __grid_const
   }
 }
 
-// ---- in place: long C2C and R2C lines (g.ip), one vector per row, a butterfly
-// per thread and stage.  A stage's rows are all read before any is written, so
+// ---- in place: long C2C and R2C lines (g.ip), a butterfly per thread and stage.  A stage's rows are all read before any is written, so
 // one row buffer serves and two CTAs fit on an SM; the lines go from memory
 // into registers, and the other CTA computes meanwhile.
 
@@ -1006,12 +1005,12 @@ __device__ __forceinline__ void rx_ip_first(const TileAddr& ta, RxV<R>* rows, co
   using Q = typename Vec<R>::Q;
   using E = std::conditional_t<KIND == P_C2C, typename Cx<R>::T, R>;
   const PassArgs& A = X.p;
-  const int m = A.m, NB = m / RAD, jb = threadIdx.x;
+  const int m = A.m, NB = m / RAD, lgG = X.g.lgG, g = threadIdx.x & ((1 << lgG) - 1), jb = threadIdx.x >> lgG;
   if (jb >= NB) return;
   constexpr int NL = Vec<R>::W * (KIND == P_C2C ? 1 : 2);  // lines of a vector
-  const E* in = reinterpret_cast<const E*>(A.in) + ta.src0;
   const long long sq = A.src_k_contig ? 1 : ta.srcq, lb = ta.srcb;
-  const int lines = ta.lines;
+  const E* in = reinterpret_cast<const E*>(A.in) + ta.src0 + g * NL * lb;
+  const int lines = ta.lines - g * NL;
   RxV<R> v[RAD];
 #pragma unroll
   for (int r = 0; r < RAD; ++r) {
@@ -1038,21 +1037,22 @@ __device__ __forceinline__ void rx_ip_first(const TileAddr& ta, RxV<R>* rows, co
         v[r] = RxV<R>{x[0], x[1]};
     }
   }
-  RxV<R>* o = rows + jb * (RAD + (X.g.pad ? 1 : 0));
-  vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r] = x; });
+  RxV<R>* o = rows + (jb * (RAD + (X.g.pad ? 1 : 0)) << lgG) + g;
+  vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r << lgG] = x; });
 }
 
 template <typename R, int RAD>
 __device__ __forceinline__ void rx_ip_mid(RxV<R>* rows, const RxArgs& X, int NS, const RxV<R>* tw, int op) {
   using Q = typename Vec<R>::Q;
-  const int NB = X.g.len / RAD, pad = X.g.pad;
-  const bool act = (int)threadIdx.x < NB;
-  const int jb = act ? threadIdx.x : NB - 1;  // idle threads read along, and write nothing
+  const int NB = X.g.len / RAD, pad = X.g.pad, lgG = X.g.lgG;
+  const bool act = (int)threadIdx.x < NB << lgG;
+  const int it = act ? threadIdx.x : 0;  // idle threads read along, and write nothing
+  const int g = it & ((1 << lgG) - 1), jb = it >> lgG;
   const unsigned mpad = pad ? fdiv_magic(pad) : 0;
-  const int rs = NB + (pad ? NB / pad : 0), ws = NS + (op ? NS / op : 0);
+  const int rs = (NB + (pad ? NB / pad : 0)) << lgG, ws = (NS + (op ? NS / op : 0)) << lgG;
   const int k = jb - (int)fdiv(jb, NS, fdiv_magic(NS)) * NS;
   RxV<R> v[RAD];
-  const RxV<R>* p = rows + rx_row(jb, pad, mpad);
+  const RxV<R>* p = rows + (rx_row(jb, pad, mpad) << lgG) + g;
 #pragma unroll
   for (int r = 0; r < RAD; ++r) v[r] = p[r * rs];
   const RxV<R>* t = tw + k;
@@ -1062,7 +1062,7 @@ __device__ __forceinline__ void rx_ip_mid(RxV<R>* rows, const RxArgs& X, int NS,
   // values of every radix alive across it
   asm volatile("bar.sync 0; // radix %0" ::"n"(RAD) : "memory");
   if (act) {
-    RxV<R>* o = rows + rx_row((jb - k) * RAD + k, op, mpad);
+    RxV<R>* o = rows + (rx_row((jb - k) * RAD + k, op, mpad) << lgG) + g;
     vb_emit<Q, RAD>(v, [&](int r, const RxV<R>& x) { o[r * ws] = x; });
   }
 }

@@ -145,12 +145,16 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
     return true;
   };
   bool ok = fits(true, false) || fits(false, false) || fits(true, true) || fits(false, true);
-  // Long lines, whose tile of the fewest sequences leaves one CTA per SM: C2C
-  // and R2C passes run in place, one butterfly per thread and stage, so that
-  // two CTAs fit and one loads while the other computes.
+  // Long lines, whose tile leaves one CTA per SM: C2C and R2C passes run in
+  // place, one butterfly per thread and stage.  With one vector per row two
+  // CTAs fit and one loads while the other computes (4096 points, direct: 1.9 ->
+  // 3.3 TB/s); a transposed C2C store takes two vectors, whose 32-byte runs are
+  // worth more than the second CTA (2.62 against 2.20 TB/s f32, 2.84 against
+  // 2.17 f64; direct 2.87 against 3.28).
+  const int wide = A.kind == P_C2C && A.dst_k_contig == 0 ? 2 : 1;
   int items = 0;
-  for (int s = 0; s < A.nstages; ++s) items = std::max(items, g->len / A.radix[s]);
-  if ((A.kind == P_C2C || A.kind == P_R2C) && !g->pre && A.nstages > 1 && G == 1 && items <= kRxMaxThreads &&
+  for (int s = 0; s < A.nstages; ++s) items = std::max(items, g->len / A.radix[s] << g->lgG);
+  if ((A.kind == P_C2C || A.kind == P_R2C) && !g->pre && A.nstages > 1 && G <= wide && G == g->P && items <= kRxMaxThreads &&
       (!ok || 2 * (g->smem + 1024) > max_smem)) {
     const int half = (max_smem - 1024) / 2;
     const int room = half - buf_bytes - tail;
