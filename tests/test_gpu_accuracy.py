@@ -41,6 +41,9 @@ def r2r(kind):
     # composite radices: the rotations inside the butterflies
     (c2c, 2048, torch.complex64, 1.685e-7), (c2c, 3000, torch.complex64, 1.816e-7),
     (c2c, 4096, torch.complex64, 1.750e-7), (c2c, 1296, torch.complex128, 3.784e-16),
+    # Bluestein's convolution lengths above 1024
+    (c2c, 521, torch.complex64, 2.236e-7), (c2c, 521, torch.complex128, 4.078e-16),
+    (c2c, 751, torch.complex64, 2.575e-7), (c2c, 1321, torch.complex64, 2.462e-7),
     (r2r("DctII"), 41, torch.float64, 3.784e-16), (r2r("DctII"), 131, torch.float64, 4.399e-16),
 ])
 def test_round_trip_error(make, n, dtype, generic):
