@@ -1442,7 +1442,10 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
         B.sub = odd_sub;
         B.m /= 2;
         B.bs_m2 = bluestein_len(B.m, P.real_bytes);
-        taken = take(B);
+        // not where the convolution is the shorter one for its points, and so the
+        // less exact one (bluestein_len): DST-I 286 f32, forward and back, 2.6e-7
+        // at 287 in 576 points, 2.1e-7 at 574 in 2048
+        if (2 * B.bs_m2 >= A.bs_m2) taken = take(B);
       }
       if (!taken) take(A);
     }

@@ -44,6 +44,8 @@ def r2r(kind):
     # Bluestein's convolution lengths above 1024
     (c2c, 521, torch.complex64, 2.236e-7), (c2c, 521, torch.complex128, 4.078e-16),
     (c2c, 751, torch.complex64, 2.575e-7), (c2c, 1321, torch.complex64, 2.462e-7),
+    # a type-I kind whose N-point form would take a shorter convolution
+    (r2r("DstI"), 286, torch.float32, 2.198e-7),
     (r2r("DctII"), 41, torch.float64, 3.784e-16), (r2r("DctII"), 131, torch.float64, 4.399e-16),
 ])
 def test_round_trip_error(make, n, dtype, generic):
