@@ -33,6 +33,14 @@ __device__ __forceinline__ bool pb_rejected(const int* gate) {
   return *reinterpret_cast<const volatile int*>(gate) != 0;
 }
 
+// An error that the caller returns, taken off the runtime's record: left there,
+// the next call that ends in cudaGetLastError (a launch with <<<>>>, the host
+// program's own check) would report it for work that was fine.
+inline cudaError_t pb_reported(cudaError_t err) {
+  if (err != cudaSuccess) (void)cudaGetLastError();
+  return err;
+}
+
 // cudaFuncAttributeMaxDynamicSharedMemorySize of KERN, set once per device.
 template <auto KERN>
 inline cudaError_t pb_allow_smem(int bytes) {
@@ -42,7 +50,7 @@ inline cudaError_t pb_allow_smem(int bytes) {
   if (err != cudaSuccess) return err;
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
   if (bit != 0 && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
-  err = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  err = pb_reported(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   if (err == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
   return err;
 }
@@ -65,7 +73,7 @@ inline cudaError_t pb_launch(void (*kern)(const Args), long long grid, int threa
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = known && capturing == cudaStreamCaptureStatusNone ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args);
+  return pb_reported(cudaLaunchKernelEx(&cfg, kern, args));
 }
 
 }  // namespace pb
