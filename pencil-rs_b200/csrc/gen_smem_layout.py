@@ -41,7 +41,7 @@ MR = [35, 36, 40, 42, 45, 48, 49, 50, 54, 56, 60, 63, 70, 72, 75, 80, 81, 84, 90
       980, 1000, 1008]
 # the mixed-radix kernel also runs the real-to-real kinds on powers of two and
 # on 770 (mr_lengths.hpp, kMrR2rLengths)
-MR_ALL = sorted(MR + [32, 64, 128, 256, 385, 512, 770])
+MR_ALL = sorted(MR + [32, 64, 128, 256, 512, 770])
 SHIFTS = [0, 2, 3, 4, 5]
 KINDS = [("c2c", False), ("r2c", False), ("c2r", False), ("c2c", True), ("r2c", True), ("c2r", True)]
 
@@ -184,7 +184,7 @@ def mr_factor(N, max_radix=16):
 
 
 def mr_nseq(N, rb):
-    fit = (3084 if rb == 4 else 1542) // N
+    fit = (3072 if rb == 4 else 1536) // N
     if fit >= 64:
         return 64
     if rb == 4 and N > 512:

@@ -129,9 +129,7 @@ __host__ __device__ constexpr int mr_tw_off(const RadixList& L, int ST) {
 template <typename R, int N, int S = 0>
 struct MRGeom {
   static constexpr int TILE_ELEMS = sizeof(R) == 4 ? 3072 : 1536;
-  // sequences that fit, with 1/256 of slack (eight of 385 points, the FFT of a
-  // 384-point DST-I)
-  static constexpr int FIT = (TILE_ELEMS + TILE_ELEMS / 256) / N;
+  static constexpr int FIT = TILE_ELEMS / N;
   // lengths above 512 (the 770-point DST-I FFT) would get 2 sequences, whose
   // transposed store writes 16-byte runs per destination row: f32 takes 4
   static constexpr int NSEQ = FIT >= 64 ? 64

@@ -73,8 +73,8 @@ constexpr int MR_GROUPS = 8;
 // Convolution lengths of Bluestein passes up to 1024 points: the smallest entry
 // >= 2m - 1 is taken (powers of two and 7-smooth lengths between them, so
 // that the convolution stays within about 1.8x of 2m); mr_bs.cuh is
-// instantiated for each.  Longer convolutions (generic kernel only) are powers
-// of two.
+// instantiated for each.  Longer ones (on the runtime-radix kernel) are powers of
+// two.
 constexpr int kBluesteinLengths[] = {80,  96,  112, 128, 160, 192, 224, 256, 288,
                                      320, 384, 448, 512, 576, 640, 768, 896, 1024};
 constexpr int kBluesteinCount = sizeof(kBluesteinLengths) / sizeof(kBluesteinLengths[0]);
@@ -89,14 +89,13 @@ constexpr int kBatchMrLengths[] = {32,  35,  36,  40,  42,  45,  48,  49,  50,  
 constexpr int kBatchMrCount = sizeof(kBatchMrLengths) / sizeof(kBatchMrLengths[0]);
 
 // FFT lengths of the real-to-real kinds on the mixed-radix kernel
-// (mr_r2r.cuh): the mixed-radix lengths, the powers of two 32..512, 385 (the
-// odd-N form of the DST-I of a 384-point axis; radix 11) and 770.
+// (mr_r2r.cuh): the mixed-radix lengths, the powers of two 32..512, and 770
+// (= 2(384 + 1), the DST-I extension of a 384-point axis; radix 11).
 constexpr int kMrR2rLengths[] = {32,  35,  36,  40,  42,  45,  48,  49,  50,  54,  56,  60,  63,  64,  70,  72,  75,
                                  80,  81,  84,  90,  96,  98,  100, 105, 108, 112, 120, 125, 126, 128, 135, 140, 144,
                                  147, 150, 160, 162, 168, 175, 180, 189, 192, 196, 200, 210, 216, 224, 225, 240, 243,
                                  245, 250, 252, 256, 270, 280, 288, 294, 300, 315, 320, 324, 336, 343, 350, 360, 375,
-                                 378, 384, 385, 392, 400, 405, 420, 432, 441, 448, 450, 480, 486, 490, 500, 504, 512,
-                                 770};
+                                 378, 384, 392, 400, 405, 420, 432, 441, 448, 450, 480, 486, 490, 500, 504, 512, 770};
 constexpr int kMrR2rCount = sizeof(kMrR2rLengths) / sizeof(kMrR2rLengths[0]);
 
 // Entry points of one (precision, length) instantiation.

@@ -1206,18 +1206,17 @@ static void build_fast_tables(pb_plan& P, PassArgs& A, const Pencil& src, const 
 
 // Whether the register kernel runs a type-I kind of 2N points (N odd) in its
 // N-point form: where that is the only one it has; in f64 where it saves a
-// stage (2N = 770: 4 stages, N = 385: 3, DST-I 384 1.14 -> 1.35 TB/s; at equal
-// counts it lost 4-19%); in f32 at equal counts where the 2N-point schedule
-// has a radix of 14 or more, which spills (DCT-I 106 0.98 -> 1.38 TB/s, DST-I 62
-// 1.20 -> 1.44, 48 1.16 -> 1.45; with smaller radices it lost up to 31%), and for
-// real data of 11 or more (DST-I 384 0.94 -> 0.98; complex 1.11 -> 1.04).
-static bool odd_form_pays(int m, int real_bytes, bool complex_data) {
+// stage (at equal counts it lost 4-19%); in f32 at equal counts where the
+// 2N-point schedule has a radix of 14 or more, which spills (DCT-I 106 0.98 ->
+// 1.38 TB/s, DST-I 62 1.20 -> 1.44, 48 1.16 -> 1.45; with smaller radices it lost
+// up to 31%).
+static bool odd_form_pays(int m, int real_bytes) {
   if (!mr_r2r_supported(m / 2, real_bytes)) return false;
   if (!mr_r2r_supported(m, real_bytes)) return true;
   int full[12], half[12];
   const int nf = mr_r2r_radices(m, real_bytes, full, 12), nh = mr_r2r_radices(m / 2, real_bytes, half, 12);
   if (real_bytes == 8) return nh < nf;
-  return nh == nf && *std::max_element(full, full + nf) >= (complex_data ? 14 : 11);
+  return nh == nf && *std::max_element(full, full + nf) >= 14;
 }
 
 // One fused pass for `st` under `op` from layout `src` to layout `dst`.
@@ -1371,7 +1370,7 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
                       : op.sub == S_DCT1                          ? S_DCT1_ODD
                                                                   : -1;
   const bool iv4 = op.sub == S_DCT4 || op.sub == S_DST4;
-  const bool odd1 = odd_sub >= 0 && odd_form_pays(A.m, P.real_bytes, in_complex);
+  const bool odd1 = odd_sub >= 0 && odd_form_pays(A.m, P.real_bytes);
   if (!A.fast && !P.force_generic && op.kind == P_R2R && (!iv4 || A.n % 2 == 0) &&
       (odd1 || mr_r2r_supported(A.m, P.real_bytes)) && (src.perm[N - 1] == a || r2r_strided) && src.split_of(a) < 0) {
     const bool direct = dst.perm[N - 1] == a && dst.split_of(a) < 0;

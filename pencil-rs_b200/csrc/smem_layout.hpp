@@ -98,7 +98,6 @@ __host__ __device__ constexpr SmemLayout mr_layout(int N, int real_bytes) {
     case 375: return real_bytes == 4 ? SmemLayout{0, 378} : SmemLayout{0, 378};
     case 378: return real_bytes == 4 ? SmemLayout{0, 378} : SmemLayout{0, 378};
     case 384: return real_bytes == 4 ? SmemLayout{0, 386} : SmemLayout{0, 386};
-    case 385: return real_bytes == 4 ? SmemLayout{0, 398} : SmemLayout{0, 390};
     case 392: return real_bytes == 4 ? SmemLayout{0, 396} : SmemLayout{0, 396};
     case 400: return real_bytes == 4 ? SmemLayout{4, 428} : SmemLayout{3, 452};
     case 405: return real_bytes == 4 ? SmemLayout{0, 412} : SmemLayout{0, 412};

@@ -1,0 +1,37 @@
+"""Which kernel and FFT length the real-to-real kinds get: step_configs of the
+first axis of an n x 4 field."""
+
+import numpy as np
+import pytest
+
+import pencil_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():  # pragma: no cover
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+import pencil_b200 as pb  # noqa: E402
+from pencil_b200 import _lib as L  # noqa: E402
+from test_gpu_parity import check_transform, rand_field  # noqa: E402
+
+
+def r2r_plan(kind, n, dtype):
+    return pb.R2rPlan.from_shape(pb.MpiTopology((1,)), (n, 4), (3,), [kind, "Dht"], dtype=dtype)
+
+
+@pytest.mark.parametrize("kind,n,dtype,kernel,fft_len", [
+    # type I, 2N-point form: where the N-point one saves nothing or has no kernel
+    ("DstI", 384, torch.float32, "mixed_radix", 770), ("DstI", 384, torch.float64, "mixed_radix", 770),
+    ("DstI", 384, torch.complex64, "mixed_radix", 770), ("DctI", 106, torch.float64, "mixed_radix", 210),
+    ("DstI", 124, torch.float32, "mixed_radix", 250),
+    # N-point form: fewer stages in f64, radix 14 or 15 avoided in f32, runtime radices
+    ("DstI", 124, torch.float64, "mixed_radix", 125), ("DctI", 106, torch.float32, "mixed_radix", 105),
+    ("DstI", 350, torch.float32, "runtime_radix", 351), ("DctI", 456, torch.float64, "runtime_radix", 455),
+    # Bluestein: the N-point form unless its convolution is the relatively shorter one
+    ("DstI", 100, torch.float32, "bluestein", 101), ("DstI", 286, torch.float32, "bluestein", 574),
+])
+def test_kernel_and_length(kind, n, dtype, kernel, fft_len):
+    c = r2r_plan(kind, n, dtype).step_configs(L.FORWARD)[-1]
+    assert (c["kernel"], c["fft_len"]) == (kernel, fft_len)
