@@ -1371,8 +1371,11 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
                                                                   : -1;
   const bool iv4 = op.sub == S_DCT4 || op.sub == S_DST4;
   const bool odd1 = odd_sub >= 0 && odd_form_pays(A.m, P.real_bytes);
+  // its row tables hold every output of a line (not those of the type-IV kinds of
+  // 1540 points on the 770-point FFT)
   if (!A.fast && !P.force_generic && op.kind == P_R2R && (!iv4 || A.n % 2 == 0) &&
-      (odd1 || mr_r2r_supported(A.m, P.real_bytes)) && (src.perm[N - 1] == a || r2r_strided) && src.split_of(a) < 0) {
+      (odd1 || mr_r2r_supported(A.m, P.real_bytes)) && A.n_out <= mr_r2r_table_len(odd1 ? A.m / 2 : A.m) &&
+      (src.perm[N - 1] == a || r2r_strided) && src.split_of(a) < 0) {
     const bool direct = dst.perm[N - 1] == a && dst.split_of(a) < 0;
     const int ta = dst.split_of(a);
     const bool transposed = !direct && dst.perm[N - 1] == b && (ta < 0 || dst.grid[ta] <= 64);
@@ -1463,16 +1466,8 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
       A.lines = L;
     }
   }
-  // the register kernels' row tables hold A.m outputs per line
-  // (mr_r2r_table_len in the real-to-real kernel): anything longer stays on
-  // the generic kernel
-  if (A.fast && A.fast != 5 && A.n_out > (A.fast == 3 ? mr_r2r_table_len(A.m) : (A.half ? 2 * A.m : A.m))) {
-    A.fast = 0;
-    A.half = 0;
-    A.m = fft_len(op.kind, op.sub, A.n);
-    A.twiddle = enc(roots_table(P, A.m));
-    A.dst_k_contig = (dst.perm[N - 1] == a) ? 1 : 0;
-  }
+  // the row tables of the C2C, R2C and C2R kernels hold A.m outputs per line
+  if ((A.fast == 1 || A.fast == 2 || A.fast == 4) && A.n_out > (A.half ? 2 * A.m : A.m)) fail(PB_EUNSUPPORTED);
   if (!A.fast) L = choose_lines(P, A, pair_kind ? 1 : 0);
   if (!A.fast && P.force_generic) {
     auto it = P.tuned_lines.find(pass_key(A, P.real_bytes));

@@ -35,3 +35,17 @@ def r2r_plan(kind, n, dtype):
 def test_kernel_and_length(kind, n, dtype, kernel, fft_len):
     c = r2r_plan(kind, n, dtype).step_configs(L.FORWARD)[-1]
     assert (c["kernel"], c["fft_len"]) == (kernel, fft_len)
+
+
+@pytest.mark.parametrize("kind", ["DctIV", "DstIV"])
+@pytest.mark.parametrize("rb,dtype", [(4, torch.float32), (8, torch.float64)])
+def test_type_four_longer_than_the_row_tables(kind, rb, dtype):
+    """A 770-point FFT with 1540 outputs per line, more than the compiled
+    kernel's row tables hold: the runtime-radix kernel's."""
+    plan = r2r_plan(kind, 1540, dtype)
+    c = plan.step_configs(L.FORWARD)[-1]
+    assert (c["kernel"], c["fft_len"]) == ("runtime_radix", 770)
+    route = po.r2r_route(po.Topology((1,)), (1540, 4), [kind, "Dht"], True)
+    x = rand_field(np.random.default_rng(35), (1540, 4), (3,), False, rb)
+    for d in ("fwd", "inv", "bwd"):
+        check_transform(plan, route, x, 3, rb, False, d)
