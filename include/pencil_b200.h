@@ -422,13 +422,18 @@ int pb_pointwise(int32_t op, int32_t scalar, const pb_pencil_desc* pencil, int32
  * runs forward_many as a sequential loop over arrays of ONE plan.  A batch here
  * holds any number of plans of one precision (different shapes, extras and
  * layouts) and an operation chain (e.g. FORWARD then INVERSE).  One execution
- * is one CUDA graph launch on a non-default stream, in one of two modes:
+ * is one CUDA graph launch (on the legacy default stream, which cannot be
+ * captured, plain launches), in one of two modes:
  *  - PB_BATCH_QUEUE: ONE persistent kernel over a level-ordered (plan, pass,
  *    tile) work queue with bounded dependency waits; tile heights chosen by an
  *    autotuner that caches its choice per pass shape;
  *  - PB_BATCH_BRANCHES (the default, 2 branches): the member plans' own pass
- *    kernels, the plans split over parallel graph branches balanced by bytes
- *    (largest first), each plan's chain in order on its branch.
+ *    kernels, the plans split over parallel branches balanced by bytes (largest
+ *    first), each plan's chain in order on its branch.  If a plan writes memory
+ *    that another plan of the batch reads or writes (one plan's result as
+ *    another's input, an array shared by two plans), the plans run one after
+ *    another in the order of `plans` instead.
+ * In queue mode the plans must be independent of one another.
  * With `autotune` set, creation also tunes the member plans' register passes
  * (pb_plan_autotune; the choices are cached per pass shape, persisted in the
  * file named by PB_TUNE_CACHE when set).  Plans whose chain needs the C2R

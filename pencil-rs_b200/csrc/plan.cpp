@@ -3351,6 +3351,7 @@ struct pb_batch {
   int branches = 2;
   std::vector<int> ops;
   std::vector<long long> weight;    // elements moved by each plan's op chain
+  std::vector<size_t> set_bytes;    // bytes of plan i's buffer of set k, at k * count + i
   std::vector<int> branch_of;       // plan -> branch
   std::vector<size_t> branch_off;   // workspace offset of each branch
   size_t branch_bytes = 0;          // workspace of all branches
@@ -3673,6 +3674,19 @@ static pb_batch* batch_create(pb_plan* const* plans, int count, const int* ops, 
       w += (long long)p.prog[user_mode(p, ops[k])].steps.size() * (p.fin.total(p.extra) + p.fout.total(p.extra));
     B->weight.push_back(w);
   }
+  B->set_bytes.assign((size_t)(nops + 1) * count, 0);
+  for (int i = 0; i < count; ++i) {
+    const pb_plan& p = *B->plans[i];
+    const size_t ends[2] = {(size_t)p.fin.total(p.extra) * p.real_bytes * (p.fin_complex ? 2 : 1),
+                            (size_t)p.fout.total(p.extra) * p.real_bytes * (p.fout_complex ? 2 : 1)};
+    for (int k = 0; k < nops; ++k) {
+      const int mode = user_mode(p, ops[k]);
+      const int fwd = mode == M_F || mode == M_FS || mode == M_AB || mode == M_AI;
+      size_t& in = B->set_bytes[(size_t)k * count + i];
+      in = std::max(in, ends[fwd ? 0 : 1]);
+      B->set_bytes[(size_t)(k + 1) * count + i] = ends[fwd ? 1 : 0];
+    }
+  }
   batch_assign_branches(*B);
   if (autotune)
     for (pb_plan* p : B->plans) {
@@ -3714,6 +3728,58 @@ static void batch_streams(pb_batch* B, int nb) {
   }
 }
 
+// Whether a plan of the batch writes memory that another one reads or writes:
+// one pass over the buffers in order of their addresses, with the furthest end
+// so far of all of them and of the written ones, and of those of a second plan.
+static bool batch_dependent(const pb_batch& B, void* const* buffers) {
+  struct Span {
+    uintptr_t lo, hi;
+    int plan;
+    bool written;
+  };
+  struct Ends {
+    uintptr_t hi = 0, other = 0;  // the furthest end, and the furthest of a plan other than `plan`
+    int plan = -1;
+    bool meets(const Span& s) const { return (plan != s.plan ? hi : other) > s.lo; }
+    void add(const Span& s) {
+      if (s.plan == plan) {
+        hi = std::max(hi, s.hi);
+      } else if (s.hi > hi) {
+        other = hi;
+        hi = s.hi;
+        plan = s.plan;
+      } else {
+        other = std::max(other, s.hi);
+      }
+    }
+  };
+  std::vector<Span> spans;
+  for (int k = 0; k <= B.nops; ++k)
+    for (int i = 0; i < B.count; ++i) {
+      const size_t at = (size_t)k * B.count + i;
+      const uintptr_t lo = reinterpret_cast<uintptr_t>(buffers[at]);
+      if (B.set_bytes[at] > 0) spans.push_back(Span{lo, lo + B.set_bytes[at], i, k > 0});
+    }
+  std::sort(spans.begin(), spans.end(), [](const Span& a, const Span& b) { return a.lo < b.lo; });
+  Ends all, written;
+  for (const Span& s : spans) {
+    if ((s.written ? all : written).meets(s)) return true;
+    all.add(s);
+    if (s.written) written.add(s);
+  }
+  return false;
+}
+
+// Every plan in order on `s` itself; a status.
+static int batch_in_order(pb_batch* B, void* const* buffers, void* ws, cudaStream_t s) {
+  try {
+    for (int i = 0; i < B->count; ++i) batch_run_plan(*B, i, buffers, ws, s);
+  } catch (const PbError& e) {
+    return e.code;
+  }
+  return PB_OK;
+}
+
 // Forks the branches from `s`, enqueues each branch's plans in order and joins
 // the branches back into `s` (also after an error); a status.
 static int batch_fork_join(pb_batch* B, int nb, void* const* buffers, void* ws, cudaStream_t s) {
@@ -3749,14 +3815,16 @@ static int batch_fork_join(pb_batch* B, int nb, void* const* buffers, void* ws, 
 // Branch mode: the branches run a share of the plans each with their own pass
 // kernels, forked from and joined back into `s`: one graph, replayed while the
 // buffers stay bound, or plain launches on the legacy default stream, which
-// cannot be captured (64 grids: 6.3 ms in order, 4.8 ms on two branches).
+// cannot be captured (64 grids: 6.3 ms in order, 4.8 ms on two branches).  Plans
+// that depend on one another through their buffers run one after another.
 static int batch_execute_branches(pb_batch* B, void* const* buffers, void* ws, cudaStream_t s) {
   const int nb = (int)B->branch_off.size();
   if (reinterpret_cast<uintptr_t>(ws) % 256 != 0) fail(PB_EINVALID_ARGUMENT);
   std::lock_guard<std::mutex> lock(B->enqueue);
   if (s == nullptr) {
     batch_streams(B, nb);
-    const int rc = batch_fork_join(B, nb, buffers, ws, s);
+    const int rc =
+        batch_dependent(*B, buffers) ? batch_in_order(B, buffers, ws, s) : batch_fork_join(B, nb, buffers, ws, s);
     if (rc != PB_OK) fail(rc);
     return PB_OK;
   }
@@ -3768,8 +3836,9 @@ static int batch_execute_branches(pb_batch* B, void* const* buffers, void* ws, c
     B->graph = nullptr;
     B->bound.clear();
     batch_streams(B, nb);
+    const bool dependent = batch_dependent(*B, buffers);
     cuda_ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    int rc = batch_fork_join(B, nb, buffers, ws, s);
+    int rc = dependent ? batch_in_order(B, buffers, ws, s) : batch_fork_join(B, nb, buffers, ws, s);
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(s, &g);
     if (rc == PB_OK && ec != cudaSuccess) rc = PB_ECUDA;

@@ -684,9 +684,11 @@ class PlanBatch:
     the same launch.  ``mode``:
 
     * ``"branches"`` (default): the plans' own pass kernels, the plans spread
-      over ``branches`` parallel graph branches balanced by bytes;
+      over ``branches`` parallel branches balanced by bytes; one after another
+      if a plan writes memory that another one reads or writes;
     * ``"queue"``: one persistent kernel over a level-ordered (plan, pass,
-      tile) work queue with bounded dependency waits.
+      tile) work queue with bounded dependency waits; the plans must be
+      independent of one another.
 
     ``autotune`` tunes the generic tile heights of the queue and the member
     plans' register passes (cached per pass shape).
