@@ -3521,6 +3521,24 @@ static void batch_assign_branches(pb_batch& B) {
   B.branch_bytes = off;
 }
 
+// The streams and events of the branches, made when the branches are chosen: an
+// execution on a new batch costs what a repeated one does.
+static void batch_streams(pb_batch& B) {
+  const size_t nb = B.branch_off.size();
+  B.bstreams.reserve(nb);
+  B.bevents.reserve(nb + 1);
+  while (B.bstreams.size() < nb) {
+    cudaStream_t st;
+    cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    B.bstreams.push_back(st);
+  }
+  while (B.bevents.size() < nb + 1) {
+    cudaEvent_t e;
+    cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    B.bevents.push_back(e);
+  }
+}
+
 static pb_batch* batch_create(pb_plan* const* plans, int count, const int* ops, int nops, int autotune) {
   if (!plans || !ops || count <= 0 || nops <= 0) fail(PB_EINVALID_ARGUMENT);
   std::unique_ptr<pb_batch> B(new pb_batch());
@@ -3688,6 +3706,7 @@ static pb_batch* batch_create(pb_plan* const* plans, int count, const int* ops, 
     }
   }
   batch_assign_branches(*B);
+  batch_streams(*B);
   if (autotune)
     for (pb_plan* p : B->plans) {
       const int rc = autotune_plan(p);
@@ -3710,21 +3729,6 @@ static void batch_run_plan(pb_batch& B, int i, void* const* buffers, void* ws, c
     void* out = buffers[(size_t)(k + 1) * B.count + i];
     const int rc = run(B.plans[i], B.ops[k], in, out, bws, st, nullptr, 0, nullptr);
     if (rc != PB_OK) fail(rc);
-  }
-}
-
-// Branch mode: one graph whose branches each run a share of the plans with
-// their own pass kernels; forked from and joined back into `s`.
-static void batch_streams(pb_batch* B, int nb) {
-  for (int b = (int)B->bstreams.size(); b < nb; ++b) {
-    cudaStream_t st;
-    cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    B->bstreams.push_back(st);
-  }
-  while ((int)B->bevents.size() < nb + 1) {
-    cudaEvent_t e;
-    cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    B->bevents.push_back(e);
   }
 }
 
@@ -3785,6 +3789,7 @@ static int batch_in_order(pb_batch* B, void* const* buffers, void* ws, cudaStrea
 static int batch_fork_join(pb_batch* B, int nb, void* const* buffers, void* ws, cudaStream_t s) {
   int forked = 0;
   int rc = PB_OK;
+  std::vector<int> next(nb, 0);
   try {
     cuda_ok(cudaEventRecord(B->bevents[0], s));
     for (int b = 0; b < nb; ++b) {
@@ -3792,7 +3797,6 @@ static int batch_fork_join(pb_batch* B, int nb, void* const* buffers, void* ws, 
       ++forked;
     }
     // the branches' plans in turn, so that a plain enqueue feeds them evenly
-    std::vector<int> next(nb, 0);
     for (int left = B->count; left > 0;) {
       for (int b = 0; b < nb; ++b) {
         while (next[b] < B->count && B->branch_of[next[b]] != b) ++next[b];
@@ -3822,7 +3826,6 @@ static int batch_execute_branches(pb_batch* B, void* const* buffers, void* ws, c
   if (reinterpret_cast<uintptr_t>(ws) % 256 != 0) fail(PB_EINVALID_ARGUMENT);
   std::lock_guard<std::mutex> lock(B->enqueue);
   if (s == nullptr) {
-    batch_streams(B, nb);
     const int rc =
         batch_dependent(*B, buffers) ? batch_in_order(B, buffers, ws, s) : batch_fork_join(B, nb, buffers, ws, s);
     if (rc != PB_OK) fail(rc);
@@ -3835,7 +3838,6 @@ static int batch_execute_branches(pb_batch* B, void* const* buffers, void* ws, c
     if (B->graph) cudaGraphExecDestroy(B->graph);
     B->graph = nullptr;
     B->bound.clear();
-    batch_streams(B, nb);
     const bool dependent = batch_dependent(*B, buffers);
     cuda_ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     int rc = dependent ? batch_in_order(B, buffers, ws, s) : batch_fork_join(B, nb, buffers, ws, s);
@@ -3941,10 +3943,12 @@ int pb_batch_set_mode(pb_batch* batch, int32_t mode, int32_t branches) {
     if (!batch) return (int)PB_ENULL;
     if ((mode != PB_BATCH_QUEUE && mode != PB_BATCH_BRANCHES) || (mode == PB_BATCH_BRANCHES && (branches < 1 || branches > 16)))
       return (int)PB_EINVALID_ARGUMENT;
+    std::lock_guard<std::mutex> lock(batch->enqueue);
     batch->mode = mode;
     if (mode == PB_BATCH_BRANCHES) {
       batch->branches = branches;
       batch_assign_branches(*batch);
+      batch_streams(*batch);
     }
     // the next execution captures (and, in queue mode, uploads its descriptors) again
     if (batch->graph) cudaGraphExecDestroy(batch->graph);

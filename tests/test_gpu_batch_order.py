@@ -1,5 +1,7 @@
-"""Branch mode with plans that share buffers, and one batch run by two threads."""
+"""Branch mode with plans that share buffers, one batch run by two threads, and
+what a first execution creates."""
 
+import ctypes as C
 import threading
 
 import pytest
@@ -120,3 +122,36 @@ def test_two_threads_run_one_batch(side_stream):
     for t in threads:
         t.join()
     assert errors == []
+
+
+def stream_ids(count):
+    """Ids of newly made streams: consecutive where nobody else makes one."""
+    cu, ids = C.CDLL("libcuda.so.1"), []
+    for _ in range(count):
+        st, i = C.c_void_p(), C.c_uint64()
+        assert cu.cuStreamCreate(C.byref(st), 1) == 0
+        assert cu.cuStreamGetId(st, C.byref(i)) == 0
+        assert cu.cuStreamDestroy_v2(st) == 0
+        ids.append(i.value)
+    return ids
+
+
+def test_a_first_execution_makes_no_streams():
+    plans = make_plans(SHAPES)
+    xs = [field(p) for p in plans]
+    outs = [p.allocate_output() for p in plans]
+    for p, x, o in zip(plans, xs, outs):
+        p.forward(x, o)
+    batch = pb.PlanBatch(plans, ("forward",), autotune=False)
+    ws = batch.allocate_workspace()
+    torch.cuda.synchronize()
+    a, b, c = stream_ids(3)
+    assert c - b == b - a
+    run(batch, [xs, outs], ws, None)
+    (d,) = stream_ids(1)
+    assert d - c == b - a
+    batch.set_mode("branches", 5)  # made here
+    (e,) = stream_ids(1)
+    run(batch, [xs, outs], batch.allocate_workspace(), None)
+    (f,) = stream_ids(1)
+    assert e - d > b - a and f - e == b - a
