@@ -988,11 +988,11 @@ static LocalOp local_op(const Stage& st, int mode, long long n_axis) {
 
 static int choose_lines_capped(pb_plan& P, PassArgs& A, int pair_kind, int cap);
 
-// Shape key of a generic pass (the autotuner's cache key).
 static cudaError_t launch_step(const PassArgs& A, int real_bytes, cudaStream_t stream) {
   return A.fast == 5 ? launch_rx(A, real_bytes, stream) : launch_pass(A, real_bytes, stream);
 }
 
+// Shape key of a generic pass (the autotuner's cache key).
 static std::string pass_key(const PassArgs& A, int real_bytes) {
   return "k" + std::to_string(A.kind) + "s" + std::to_string(A.sub) + "n" + std::to_string(A.n_in) + "o" +
          std::to_string(A.n_out) + "m" + std::to_string(A.m) + "r" + std::to_string(real_bytes) + "c" +

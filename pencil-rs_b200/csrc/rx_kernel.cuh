@@ -19,7 +19,7 @@
 //
 //   first stage   staged lines -> butterfly -> rows (or, with `pre`, a pass
 //                 that forms the rows: the real-to-real kinds' reordering and
-//                 pre-twiddles, and lengths with a prime above 16)
+//                 pre-twiddles, and lengths with a prime above 23)
 //   middle stages rows -> rows, alternating between two buffers
 //   last stage    C2C: butterfly outputs go to memory from registers; the
 //                 other kinds read the finished rows back (the Hermitian
@@ -31,10 +31,11 @@
 // Inverse transforms read their input in reversed index order, X^-1[k] =
 // DFT(x[-q])[k], so only forward butterflies exist.
 //
-// What bounds it: shared-memory and barrier latency at 12 to 16 warps per SM,
-// not HBM (ncu, 384-point C2C f32: DRAM 55%, issue 45%, LSU data pipe 63%).
+// What bounds it: global- and shared-memory latency and barriers at 16 warps per
+// SM, not HBM (ncu: 255-point C2C f64 DRAM 24-30%, issue 33-36%, LSU data pipe
+// 32-40%; 4096-point C2C f32 24-29%, 36-39%, 36-42%).
 // Against the generic kernel on the same passes (B200, forward + inverse):
-// 255^3 R2C f64 3.43 -> 1.11 ms, 4096^2 C2C f32 2.30 -> 0.63 ms; single
+// 255^3 R2C f64 3.43 -> 0.76 ms, 4096^2 C2C f32 2.30 -> 0.40 ms; single
 // transposed C2C passes run at 2.4-3.9 TB/s.  Measured choices: tiles of about
 // 2000 points with 128 threads and four CTAs per SM beat tiles of twice the
 // lines with 256 threads (384 points: 3.9 against 3.1 TB/s); 80 registers and

@@ -9,10 +9,9 @@
 
 namespace pb {
 
-std::vector<int> rx_radices(int m, int real_bytes) {
-  (void)real_bytes;
+std::vector<int> rx_radices(int m) {
   static const int radices[] = {31, 29, 23, 19, 17, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-  if (m < 2) return m == 1 ? std::vector<int>{} : std::vector<int>{};
+  if (m < 2) return {};
   // fewest stages, then the smallest largest radix, over the divisors of m
   constexpr int kInf = 1 << 20;
   std::vector<int> st(m + 1, kInf), mx(m + 1, 0), ch(m + 1, 0);
@@ -175,7 +174,7 @@ bool rx_geometry(const PassArgs& A, int real_bytes, int max_smem, RxGeom* g) {
 
 bool rx_choose(PassArgs& A, int real_bytes, int max_smem, long long max_chunk, long long total_lines, int sms) {
   const int len = A.bs_m2 ? A.bs_m2 : A.m;
-  const std::vector<int> rad = rx_radices(len, real_bytes);
+  const std::vector<int> rad = rx_radices(len);
   if (rad.empty()) return false;
   A.nstages = (int)rad.size();
   for (int s = 0; s < A.nstages; ++s) A.radix[s] = rad[s];

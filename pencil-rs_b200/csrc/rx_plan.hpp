@@ -46,7 +46,7 @@ struct RxArgs {
 
 // Stage radices of an m-point transform (stage 0 first); empty when m has a
 // prime factor above 31.
-std::vector<int> rx_radices(int m, int real_bytes);
+std::vector<int> rx_radices(int m);
 
 // The per-stage twiddle table of a radix list: for stage s the (R-1)*NS
 // entries W^{k r} of a (NS*R)-point transform, then for a prime radix above
