@@ -52,18 +52,6 @@ int bs_lines_r(int M) {
     return 0;
   }
 }
-
-template <typename R, int I = 0>
-int bs_radices_r(int M, int* radices, int cap) {
-  if constexpr (I < kBluesteinCount) {
-    constexpr RadixList L = MRGeom<R, kBluesteinLengths[I]>::RL;
-    if (M != kBluesteinLengths[I]) return bs_radices_r<R, I + 1>(M, radices, cap);
-    for (int i = 0; i < L.n && i < cap; ++i) radices[i] = L.r[i];
-    return L.n;
-  } else {
-    return 0;
-  }
-}
 #endif
 
 }  // namespace
@@ -87,10 +75,6 @@ bool mr_bs_supported(int M, int real_bytes) {
 }
 
 int mr_bs_lines(int M, int real_bytes) { return real_bytes == 4 ? bs_lines_r<float>(M) : bs_lines_r<double>(M); }
-
-int mr_bs_radices(int M, int real_bytes, int* radices, int cap) {
-  return real_bytes == 4 ? bs_radices_r<float>(M, radices, cap) : bs_radices_r<double>(M, radices, cap);
-}
 
 int mr_bs_occupancy(int M, int kind, int variant, int real_bytes) {
   const bool c2c = kind == P_C2C;

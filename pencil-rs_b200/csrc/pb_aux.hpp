@@ -126,7 +126,6 @@ int mr_r2r_occupancy(int m, int real_bytes);
 bool mr_bs_supported(int M, int real_bytes);
 cudaError_t launch_mr_bs(const PassArgs& A, int real_bytes, cudaStream_t stream);
 int mr_bs_lines(int M, int real_bytes);
-int mr_bs_radices(int M, int real_bytes, int* radices, int cap);  // stage radices, stage 0 first; their number
 int mr_bs_occupancy(int M, int kind, int variant, int real_bytes);
 // the layout variant of a Bluestein pass: 0 contiguous lines, 1 strided
 // lines, 2 contiguous lines with a split direct store

@@ -4715,9 +4715,12 @@ int pb_plan_step_config(const pb_plan* plan, int32_t op, int32_t step, pb_step_c
       out->nradix = mr_r2r_radices(A.m, plan->real_bytes, out->radix, 12);
     else if (A.fast == 1)
       out->nradix = pow2_radices(A.m, out->radix, 12);
-    else if (A.fast == 4)
-      out->nradix = mr_bs_radices(A.bs_m2, plan->real_bytes, out->radix, 12);
-    else {
+
+    else if (A.bs_m2) {  // the convolution length, as its prime-power factors
+      const std::vector<int> r = radices(A.bs_m2);
+      out->nradix = std::min((int)r.size(), 12);
+      for (int i = 0; i < out->nradix; ++i) out->radix[i] = r[i];
+    } else {
       out->nradix = std::min(A.nstages, 12);
       for (int i = 0; i < out->nradix; ++i) out->radix[i] = A.radix[i];
     }

@@ -324,10 +324,10 @@ class _Plan:
 
     def step_kernels(self, op) -> list:
         """Kernel family of each launch of one operation: "generic", "check",
-        "pow2" (register-resident power-of-two pass), "mixed_radix",
-        "bluestein" (a length with a prime factor above 31, on the mixed-radix
-        or the runtime-radix kernel) or "runtime_radix" (other lengths with
-        prime factors up to 31)."""
+        "pow2" (register-resident power-of-two pass), "mixed_radix" or
+        "bluestein" (a C2C / R2C / C2R length with a prime factor above 31 on
+        the mixed-radix kernel) or "runtime_radix" (other lengths with prime
+        factors up to 31)."""
         cap = 64
         ks = (C.c_int32 * cap)()
         cnt = C.c_int32()

@@ -49,19 +49,3 @@ def test_type_four_longer_than_the_row_tables(kind, rb, dtype):
     x = rand_field(np.random.default_rng(35), (1540, 4), (3,), False, rb)
     for d in ("fwd", "inv", "bwd"):
         check_transform(plan, route, x, 3, rb, False, d)
-
-
-@pytest.mark.parametrize("make,n,dtype,fft_len,radices", [
-    (pb.C2cPlan, 4096, torch.complex64, 4096, [16, 16, 16]), (pb.C2cPlan, 255, torch.complex128, 255, [15, 17]),
-    (pb.C2cPlan, 257, torch.complex64, 257, [8, 8, 9]), (pb.C2cPlan, 257, torch.complex128, 257, [4, 4, 6, 6]),
-    (pb.C2cPlan, 509, torch.complex64, 509, [4, 4, 8, 8]), (pb.C2cPlan, 521, torch.complex64, 521, [8, 16, 16]),
-    ("DstI", 100, torch.float32, 101, [14, 16]), ("DctII", 257, torch.float64, 257, [8, 8, 9]),
-])
-def test_reported_radices_are_the_kernels_own(make, n, dtype, fft_len, radices):
-    """A Bluestein pass reports the stages of its convolution."""
-    if isinstance(make, str):
-        plan = r2r_plan(make, n, dtype)
-    else:
-        plan = make.from_shape(pb.MpiTopology((1,)), (n, 4), (3,), dtype=dtype)
-    c = plan.step_configs(L.FORWARD)[-1]
-    assert (c["fft_len"], sorted(c["radices"])) == (fft_len, radices)
