@@ -210,10 +210,11 @@ int pb_plan_steps(const pb_plan* plan, int32_t op, int32_t* kinds, int32_t capac
 /* Kernel family of each launch of one operation, in order: 0 = generic fused
  * pass (shared-memory Stockham, any length and kind), 1 = C2R spectrum check,
  * 2 = register-resident power-of-two pass, 3 = register-fed mixed-radix pass
- * (7-smooth lengths), 4 = Bluestein C2C / R2C / C2R pass on the mixed-radix kernel
- * (lengths with a prime factor above 31), 5 = runtime-radix pass (the other
- * lengths with prime factors up to 31, every kind).  A diagnostic with no
- * counterpart in the reference. */
+ * (7-smooth lengths), 4 = Bluestein pass (lengths with a prime factor above 31):
+ * C2C / R2C / C2R with convolutions up to 1024 points on the mixed-radix kernel,
+ * the longer ones and the real-to-real kinds on the runtime-radix kernel, 5 =
+ * runtime-radix pass (the other lengths with prime factors up to 31, every
+ * kind).  A diagnostic with no counterpart in the reference. */
 int pb_plan_step_kernels(const pb_plan* plan, int32_t op, int32_t* kernels, int32_t capacity, int32_t* count);
 
 /* Autotuner (no counterpart in the reference, whose line FFTs are RustFFT
@@ -242,7 +243,8 @@ typedef struct pb_step_config {
   int32_t sched;      /* mixed-radix schedule */
   int32_t tuned;      /* 1: chosen by the autotuner */
   int32_t nradix;
-  int32_t radix[12];  /* stage radices, stage 0 first */
+  int32_t radix[12];  /* stage radices, stage 0 first; of a Bluestein pass the convolution
+                       * length's factors up to 8, not its kernel's stages */
 } pb_step_config;
 int pb_plan_step_config(const pb_plan* plan, int32_t op, int32_t step, pb_step_config* out);
 

@@ -324,10 +324,10 @@ class _Plan:
 
     def step_kernels(self, op) -> list:
         """Kernel family of each launch of one operation: "generic", "check",
-        "pow2" (register-resident power-of-two pass), "mixed_radix" or
-        "bluestein" (a C2C / R2C / C2R length with a prime factor above 31 on
-        the mixed-radix kernel) or "runtime_radix" (other lengths with prime
-        factors up to 31)."""
+        "pow2" (register-resident power-of-two pass), "mixed_radix",
+        "bluestein" (a length with a prime factor above 31, on the mixed-radix
+        or the runtime-radix kernel) or "runtime_radix" (other lengths with
+        prime factors up to 31)."""
         cap = 64
         ks = (C.c_int32 * cap)()
         cnt = C.c_int32()
@@ -380,8 +380,9 @@ class _Plan:
 
     def step_configs(self, op) -> list:
         """Per launch of `op`: kernel family, FFT length, lines per tile,
-        persistent grid, CTAs per SM, schedule, radices and whether the
-        autotuner chose it."""
+        persistent grid, CTAs per SM, schedule, radices (of a Bluestein pass
+        the convolution length's factors up to 8) and whether the autotuner
+        chose it."""
         names = ("generic", "check", "pow2", "mixed_radix", "bluestein", "runtime_radix")
         out = []
         for i in range(len(self.step_kinds(op))):

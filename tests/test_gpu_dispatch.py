@@ -49,3 +49,20 @@ def test_type_four_longer_than_the_row_tables(kind, rb, dtype):
     x = rand_field(np.random.default_rng(35), (1540, 4), (3,), False, rb)
     for d in ("fwd", "inv", "bwd"):
         check_transform(plan, route, x, 3, rb, False, d)
+
+
+@pytest.mark.parametrize("make,n,dtype,radices", [
+    (pb.C2cPlan, 4096, torch.complex64, [16, 16, 16]), (pb.C2cPlan, 255, torch.complex128, [15, 17]),
+    # Bluestein: 576 and 1024 points on the mixed-radix kernel, 2048 and 224 on the runtime-radix one
+    (pb.C2cPlan, 257, torch.complex64, [3, 3, 8, 8]), (pb.C2cPlan, 509, torch.complex64, [2, 8, 8, 8]),
+    (pb.C2cPlan, 521, torch.complex64, [4, 8, 8, 8]), ("DstI", 100, torch.float32, [4, 7, 8]),
+])
+def test_reported_radices(make, n, dtype, radices):
+    """The stages of a pass; of a Bluestein pass the factors of its convolution
+    length."""
+    if isinstance(make, str):
+        plan = r2r_plan(make, n, dtype)
+    else:
+        plan = make.from_shape(pb.MpiTopology((1,)), (n, 4), (3,), dtype=dtype)
+    c = plan.step_configs(L.FORWARD)[-1]
+    assert sorted(c["radices"]) == radices and (c["kernel"] == "bluestein") == (n not in (255, 4096))
