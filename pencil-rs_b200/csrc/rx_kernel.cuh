@@ -4,7 +4,7 @@
 // form of the others: two transforms of the convolution length without leaving
 // shared memory, the chirp and the kernel multiplied in as their first stages
 // read the rows.  Bluestein passes of the generic kernel ran at 0.06-0.17 TB/s
-// (DST-I 100 and 256, DCT-I 384); here 0.27-0.34, and 0.5-0.8 on DCT-II 257
+// (DST-I 100 and 256, DCT-I 384); here 0.15-0.34, and 0.5-0.8 on DCT-II 257
 // and DCT-IV 94.  C2C, R2C and C2R convolutions up to 1024 points keep the
 // compiled kernel (mr_bs.cuh), which is 1.1-1.7 times faster than this one.
 //
