@@ -66,7 +66,7 @@ __host__ __device__ constexpr int mr_r2r_min_ctas(int real_bytes, int N) {
 // Outputs per line that the real-to-real kernel's row tables hold for FFT
 // length N: 2N up to 512 (the type-IV kinds write n = 2N outputs from an
 // N-point FFT), N above (770 serves the DST-I of 384, 384 outputs).  The host
-// keeps passes with more outputs on the generic kernel.
+// gives passes with more outputs to another kernel.
 __host__ __device__ constexpr int mr_r2r_table_len(int N) { return N <= 512 ? 2 * N : N; }
 constexpr int MR_GROUPS = 8;
 

@@ -1246,7 +1246,8 @@ static Step make_pass(pb_plan& P, const Stage& st, const LocalOp& op, const Penc
   if (A.m > (1 << 20)) fail(PB_EUNSUPPORTED);
   if (op.kind != P_COPY) {
     // Bluestein: the generic kernel runs an M-point FFT (radices, roots) in
-    // place of the m-point one; the register kernels never take such lengths
+    // place of the m-point one; the register kernels that take the pass set
+    // their own below
     const int M = bluestein_len(A.m, P.real_bytes);
     auto r = radices(M ? M : A.m);
     A.nstages = (int)r.size();
